@@ -317,7 +317,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     if (c.twb < 0 || c.twb > 15) return false;
     if ((c.twb & SK_MIRROR_PAIR) && (!real_op || c.radices.size() < 2)) c.twb &= ~SK_MIRROR_PAIR;
     if ((c.twb & SK_SPLIT_PASS0) && (c.radices.size() < 2 || op == OP_PC)) c.twb &= ~SK_SPLIT_PASS0;
-    const long long buf = (long long)sk_buffer_values(op, c.P, n, r0) * 8;
+    const long long buf = (long long)sk_buffer_values(op, c.P, n, r0, c.twb) * 8;
     long long tws = (long long)sk_tws_values(op, n, c.radices.data(), (int)c.radices.size(), c.twb) * 8;
     if (buf + tws > kMaxTileSmem && (c.twb & SK_TW_SMEM)) {  // no room for the staged twiddles
         c.twb &= ~SK_TW_SMEM;

@@ -72,11 +72,16 @@ SIP_HD constexpr int sk_stage_values(int op, int p, int n) {
          : op == OP_C2R_PAIR ? p * (n + 1)
          : p * n;  // R2C pair: 2P rows of N floats = P*N complex slots
 }
+// Slots of the staging buffer: one more where the staged run may start on
+// either half of a 16-byte unit (SK_SPLIT_PASS0, sk_stage_shift).
+SIP_HD constexpr int sk_stage_slots(int op, int p, int n, int flags) {
+    return sk_stage_values(op, p, n) + ((flags & SK_SPLIT_PASS0) != 0 ? 1 : 0);
+}
 // Complex values per buffer, rounded up to an even count so that the
 // second buffer starts on a 16-byte boundary (cp.async 16-byte copies).
-SIP_HD constexpr int sk_buffer_values(int op, int p, int n, int r0) {
-    return ((sk_stage_values(op, p, n) > p * sk_pitch(n, r0) ? sk_stage_values(op, p, n) : p * sk_pitch(n, r0)) + 1) /
-           2 * 2;
+SIP_HD constexpr int sk_buffer_values(int op, int p, int n, int r0, int flags) {
+    const int stage = sk_stage_slots(op, p, n, flags), work = p * sk_pitch(n, r0);
+    return ((stage > work ? stage : work) + 1) / 2 * 2;
 }
 
 template <int N_, int P_, int T_, int OP_, int MODE_, int SIGN_, bool TW4_, int MINB_, int TWB_, int... Rs>
@@ -128,9 +133,10 @@ struct SkCfg {
     static constexpr int H = P / 2;
     static constexpr int slots(int p) { return (P * (N / radix(p)) + T - 1) / T; }
 
-    static constexpr int LD = sk_pitch(N, radix(0));
+    static constexpr int rad_list[] = {Rs...};
     static constexpr int STAGE = sk_stage_values(OP, P, N);
-    static constexpr int BUF = sk_buffer_values(OP, P, N, radix(0));
+    static constexpr int LD = sk_pitch(N, radix(0));
+    static constexpr int BUF = sk_buffer_values(OP, P, N, radix(0), FLAGS);
     // Staged twiddles (SK_TW_SMEM): per pass p with span > 1, twcount rows
     // of tws_stride(p) entries from tws_off(p), then TW2S real twiddles.
     static constexpr int tws_stride(int p) { return sk_tws_stride(CFG_OP, FLAGS, p, NP, span(p)); }
@@ -170,7 +176,6 @@ struct SkCfg {
     static_assert(!MPAIR || (OP != OP_C2R_HALF && OP != OP_C2R_PAIR) || SIGN > 0,
                   "C2R tiles run the inverse transform");
     static_assert(!SPLIT || (NP >= 2 && OP != OP_PC), "a split pass 0 needs a later pass, and no pulse tile");
-    static constexpr int rad_list[] = {Rs...};
     static_assert(TWSM == sk_tws_values(OP_, N_, rad_list, NP, TWB_), "staged twiddle layout");
 };
 
@@ -289,10 +294,111 @@ SIP_HD void sk_copy_run(int tid, int T, float2* stage_base, int stage_off_bytes,
     }
 }
 
+// One 16-byte asynchronous copy.
+SIP_HD void sk_copy16(float2* dst, const float2* src) {
+#if defined(__CUDA_ARCH__)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+#else
+    dst[0] = src[0];
+    dst[1] = src[1];
+#endif
+}
+
+SIP_HD void sk_copy8(float2* dst, const float2* src) {
+#if defined(__CUDA_ARCH__)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+#else
+    dst[0] = src[0];
+#endif
+}
+
+// The contiguous run a row tile stages: its first byte.
+template <class K>
+SIP_HD const char* sk_run_start(const TileArgs& a, const TileCtx& c) {
+    const char* src = static_cast<const char*>(a.src);
+    if constexpr (K::OP == OP_R2C_PAIR) return src + 2LL * c.i0 * a.in_idist * 4;
+    else if constexpr (K::OP == OP_C2R_PAIR) return src + 2LL * c.i0 * a.in_idist * 8;
+    else return src + c.in_base * 8;
+}
+
+// Slots (0 or 1) by which a row tile's run is shifted in its staging buffer
+// so that both sides of the copy have the same 16-byte phase: rows of an odd
+// number of complex values (C2R half spectra, row pairs, odd lengths) start
+// on either half of a 16-byte unit, and 16-byte copies would otherwise
+// fall back to 8 or 4 bytes.
+template <class K>
+SIP_HD int sk_stage_shift(const TileArgs& a, const TileCtx& c) {
+    if constexpr (K::SPLIT && K::MODE != SK_COLS && !K::MIRROR) {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(sk_run_start<K>(a, c));
+        return (p & 7) == 0 ? (int)(p >> 3) & 1 : 0;
+    }
+    return 0;
+}
+
+// `VALUES` contiguous complex values from an 8-byte aligned `src` to `dst` of
+// the same 16-byte phase (`shift`: its second half): compile-time trip counts
+// and constant address steps, one instruction per 16 bytes.  These tiles are
+// bound by instruction issue (61 % of the slots at 12 warps per SM, DRAM at
+// 48 %, for C2C rows of 4096), so what a value costs beside its arithmetic is
+// time: with this copy and the constant store addresses of store_slot
+// instead of 64-bit index products and per-value flags, C2C 8192 x 8192 went from
+// 302 to 268 us, 3840 x 8192 from 124 to 112, 65536 x 4096 from 1.82 to 1.65 ms.
+template <int VALUES, int T>
+SIP_HD void sk_copy_full(int tid, float2* dst, const float2* src, int shift) {
+    constexpr int C = (VALUES - 1) / 2;  // 16-byte units whatever the phase
+    float2* d = dst + shift + 2 * tid;
+    const float2* s = src + shift + 2 * tid;
+#pragma unroll
+    for (int i = 0; i < C / T; ++i) sk_copy16(d + 2 * i * T, s + 2 * i * T);
+    if (C % T != 0 && tid < C % T) sk_copy16(d + 2 * (C / T) * T, s + 2 * (C / T) * T);
+    // what is left: the value before them (shift) and the one or two after
+    if (tid == T - 1) {
+        if (shift) sk_copy8(dst, src);
+        if (2 * C + shift < VALUES) sk_copy8(dst + 2 * C + shift, src + 2 * C + shift);
+        if (2 * C + shift + 1 < VALUES) sk_copy8(dst + 2 * C + shift + 1, src + 2 * C + shift + 1);
+    }
+}
+
+// Full column tile: N runs of P adjacent columns, 16-byte aligned.
+template <class K>
+SIP_HD void sk_copy_full_cols(int tid, float2* dst, const float2* src, long long pitch) {
+    constexpr int CPR = K::P / 2, ROWS = K::T / CPR, T = K::T;
+    static_assert(K::P % 2 == 0 && T % CPR == 0, "whole runs per sweep of the threads");
+    const int n0 = tid / CPR, cc = tid % CPR;
+    dst += n0 * K::P + 2 * cc;
+    src += n0 * pitch + 2 * cc;
+    const long long step = ROWS * pitch;
+#pragma unroll
+    for (int i = 0; i < K::N / ROWS; ++i, src += step) sk_copy16(dst + i * ROWS * K::P, src);
+    if (K::N % ROWS != 0 && n0 < K::N % ROWS) sk_copy16(dst + (K::N / ROWS) * ROWS * K::P, src);
+}
+
 template <class K>
 SIP_HD void sk_stage(int tid, const TileArgs& a, const TileCtx& c, float2* stage) {
     constexpr int T = K::T;
     const char* src = static_cast<const char*>(a.src);
+    // Full tiles of contiguous rows or adjacent columns.
+    if constexpr (!K::MIRROR && K::MODE == SK_COLS) {
+        if constexpr (K::P % 2 == 0 && T % (K::P / 2) == 0) {
+            const float2* base = reinterpret_cast<const float2*>(src) + c.in_base;
+            const uintptr_t phase = reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(stage);
+            if (c.cnt == K::P && (phase & 15) == 0 && a.in_stride % 2 == 0) {
+                sk_copy_full_cols<K>(tid, stage, base, a.in_stride);
+                return;
+            }
+        }
+    } else if constexpr (!K::MIRROR) {
+        const float2* run = reinterpret_cast<const float2*>(sk_run_start<K>(a, c));
+        const int shift = sk_stage_shift<K>(a, c);
+        stage += shift;
+        bool full = c.cnt == K::P && !(K::OP == OP_PC && (a.flags & TF_BLUE));
+        if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) full = full && a.rows >= 2 * (c.i0 + K::P);
+        const uintptr_t phase = reinterpret_cast<uintptr_t>(run) ^ reinterpret_cast<uintptr_t>(stage);
+        if (full && (phase & 15) == 0 && (reinterpret_cast<uintptr_t>(run) & 7) == 0) {
+            sk_copy_full<K::STAGE, T>(tid, stage, run, (int)(reinterpret_cast<uintptr_t>(run) >> 3) & 1);
+            return;
+        }
+    }
     if constexpr (K::MODE == SK_COLS && !K::MIRROR) {
         // [n][q]: one run of cnt adjacent columns per element index n
         const char* base = src + c.in_base * 8;
@@ -409,6 +515,7 @@ SIP_HD void sk_zero_missing(int tid, const TileArgs& a, const TileCtx& c, float2
     if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
         const int r0 = 2 * c.i0;
         const int nrows = (a.rows - r0) < 2 * c.cnt ? (a.rows - r0) : 2 * c.cnt;
+        stage += sk_stage_shift<K>(a, c);
         if (nrows & 1) {
             if constexpr (K::OP == OP_R2C_PAIR) {
                 float* s = reinterpret_cast<float*>(stage) + (long long)nrows * K::N;
@@ -474,8 +581,8 @@ SIP_HD float2 sk_input(const TileArgs& a, const TileCtx& c, const float2* stage,
         }
         return stage[q * N + n];
     } else if constexpr (K::OP == OP_C2C) {
-        const float2 v = K::MODE == SK_COLS ? stage[n * K::P + q] : stage[q * N + n];
-        return maybe_conj(v, (a.flags & TF_CONJ_IN) != 0);
+        // (the planner conjugates the operands of real steps only)
+        return K::MODE == SK_COLS ? stage[n * K::P + q] : stage[q * N + n];
     } else if constexpr (K::OP == OP_R2C_HALF || K::OP == OP_R2C_4B) {
         return stage[q * N + n];
     } else if constexpr (K::OP == OP_C2R_4A) {
@@ -483,19 +590,6 @@ SIP_HD float2 sk_input(const TileArgs& a, const TileCtx& c, const float2* stage,
     } else if constexpr (K::OP == OP_R2C_PAIR) {
         const float* s = reinterpret_cast<const float*>(stage);
         return make_float2(s[(2 * q) * N + n], s[(2 * q + 1) * N + n]);
-    } else if constexpr (K::OP == OP_C2R_HALF) {
-        // Z[n] = E + i W_{2M}^{+n} D from X[n], X[M-n] (DC / Nyquist use real parts only)
-        const float2* row = stage + q * (N + 1);
-        const bool cj = (a.flags & TF_CONJ_IN) != 0;
-        if (n == 0) {
-            const float dc = row[0].x, ny = row[N].x;
-            return make_float2(0.5f * (dc + ny), 0.5f * (dc - ny));
-        }
-        const float2 x = maybe_conj(row[n], cj), y = maybe_conj(row[N - n], cj);
-        const float2 e = make_float2(0.5f * (x.x + y.x), 0.5f * (x.y - y.y));
-        const float2 d = make_float2(0.5f * (x.x - y.x), 0.5f * (x.y + y.y));
-        const float2 od = c_mulc(d, sk_tw2<K>(a, c, n));
-        return make_float2(e.x - od.y, e.y + od.x);
     } else {  // OP_C2R_PAIR
         constexpr int H = N / 2 + 1;
         const int kk = n <= N / 2 ? n : N - n;
@@ -538,7 +632,6 @@ struct SkPass {
     static constexpr bool COL = K::colmap(PASS);
     static constexpr bool LAST = PASS == K::NP - 1;
     using Regs = PassRegs<R, S>;
-
     SIP_HD static void butterfly_index(int b, int& q, int& j) {
         if (COL) {
             q = b % K::P;
@@ -560,23 +653,21 @@ struct SkPass {
         if constexpr (PASS == 0 && !K::WORK_IN && K::OP == OP_C2R_HALF) {
             // C2R pre-process: the twiddle of element n = j + r NR is
             // W_{2M}^{j + r NR} = W_{2M}^j W_{2R}^r, one table entry per
-            // butterfly times compile-time constants
+            // butterfly times compile-time constants.  The factors 1/2 here
+            // and 2 of the unpacked output cancel: neither is applied.
             const float2 wj = sk_tw2<K>(a, c, j);
             const float2* row = buf + q * (K::N + 1);
-            const bool cj = (a.flags & TF_CONJ_IN) != 0;
+            const float sg = (a.flags & TF_CONJ_IN) != 0 ? -1.f : 1.f;
             sk_static_for<0, R>([&](auto ic) {
                 constexpr int r = decltype(ic)::value;
                 const int n = j + r * NR;
-                if (n == 0) {
-                    const float dc = row[0].x, ny = row[K::N].x;
-                    v[r] = make_float2(0.5f * (dc + ny), 0.5f * (dc - ny));
-                } else {
-                    const float2 x = maybe_conj(row[n], cj), y = maybe_conj(row[K::N - n], cj);
-                    const float2 e = make_float2(0.5f * (x.x + y.x), 0.5f * (x.y - y.y));
-                    const float2 d = make_float2(0.5f * (x.x - y.x), 0.5f * (x.y + y.y));
-                    const float2 od = c_mulc(d, tw_const<2 * R, r, -1>(wj));
-                    v[r] = make_float2(e.x - od.y, e.y + od.x);
-                }
+                float2 x = row[n], y = row[K::N - n];
+                if (r == 0 && n == 0) x.y = y.y = 0.f;  // DC and Nyquist: real parts only
+                const float yy = sg * y.y;
+                const float2 e = make_float2(x.x + y.x, sg * x.y - yy);
+                const float2 d = make_float2(x.x - y.x, sg * x.y + yy);
+                const float2 od = c_mulc(d, tw_const<2 * R, r, -1>(wj));
+                v[r] = make_float2(e.x - od.y, e.y + od.x);
             });
         } else {
 #pragma unroll
@@ -622,50 +713,74 @@ struct SkPass {
     }
 
     // Last pass straight to global memory: element k = j + r N/R of transform q.
-    SIP_HD static void write_global(int tid, const TileArgs& a, const TileCtx& c, const Regs& rg) {
-        static_assert(LAST, "global store from the last pass only");
-        const bool sc = (a.flags & TF_SCALE) != 0;
+    // The flags are uniform branches around whole butterflies and the
+    // addresses a base plus constant steps, so that a stored value costs its
+    // store alone.
+    SIP_HD static void store_slot(int tid, int s, const TileArgs& a, const TileCtx& c, float2 (&v)[R]) {
+        const int b = tid + s * K::T;
+        if (TOTAL % K::T != 0 && b >= TOTAL) return;
+        int q, j;
+        butterfly_index(b, q, j);
+        if (!K::MIRROR && q >= c.cnt) return;
+        if constexpr (K::OP == OP_C2C) {
+            const bool blue = K::WORK_IN && (a.flags & TF_BLUE) != 0;
+            if constexpr (K::TW4) {
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            const int b = tid + s * K::T;
-            if (TOTAL % K::T == 0 || b < TOTAL) {
-                int q, j;
-                butterfly_index(b, q, j);
-                if (!K::MIRROR && q >= c.cnt) continue;
+                for (int r = 0; r < R; ++r)
+                    v[r] = c_tw<K::SIGN>(v[r], cross_tw(a, (long long)(c.i0 + q) * (j + r * NR)));
+            }
+            if (blue) {  // Bluestein: outputs k < n_other times the chirp
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const int k = j + r * NR;
-                    float2 v = rg.v[s][r];
-                    if constexpr (K::OP == OP_C2C) {
-                        if constexpr (K::WORK_IN) {  // inverse half of a pulse tile
-                            if (a.flags & TF_BLUE) {  // Bluestein: outputs k < n_other times the chirp
-                                if (k >= a.n_other) continue;
-                                v = c_mul(v, SIP_LDG(a.tw2 + k));
-                            }
-                        }
-                        if constexpr (K::TW4) v = c_tw<K::SIGN>(v, cross_tw(a, (long long)(c.i0 + q) * k));
-                        if (sc) v = c_scale(v, a.scale);
-                        v = maybe_conj(v, (a.flags & TF_CONJ_OUT) != 0);
-                        static_cast<float2*>(a.dst)[c.out_base + (long long)q * a.out_idist + (long long)k * a.out_stride] = v;
-                    } else if constexpr (K::OP == OP_C2R_4A) {
-                        const int col = sk_c2r4a_col<K>(a, c.i0, c.cnt, q);
-                        if (col < 0) continue;
-                        v = c_tw<K::SIGN>(v, cross_tw(a, 2LL * col * k));
-                        if (sc) v = c_scale(v, a.scale);
-                        static_cast<float2*>(a.dst)[c.out_base - c.i0 + col + (long long)k * a.out_stride] = v;
-                    } else if constexpr (K::OP == OP_C2R_HALF) {
-                        const float f = 2.0f * (sc ? a.scale : 1.0f);
-                        static_cast<float2*>(a.dst)[c.out_base + (long long)q * a.out_idist + k] = c_scale(v, f);
-                    } else if constexpr (K::OP == OP_C2R_PAIR) {
-                        const float f = sc ? a.scale : 1.0f;
-                        const int row = 2 * (c.i0 + q);
-                        float* d = static_cast<float*>(a.dst);
-                        d[(long long)row * a.out_idist + k] = v.x * f;
-                        if (row + 1 < a.rows) d[(long long)(row + 1) * a.out_idist + k] = v.y * f;
-                    }
-                }
+                for (int r = 0; r < R; ++r)
+                    if (j + r * NR < a.n_other) v[r] = c_mul(v[r], SIP_LDG(a.tw2 + j + r * NR));
+            }
+            if (a.flags & TF_SCALE) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = c_scale(v[r], a.scale);
+            }
+            float2* d = static_cast<float2*>(a.dst) + c.out_base + (long long)q * a.out_idist;
+            if constexpr (K::MODE == SK_ROWS) {  // out_stride is 1
+                d += j;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (!blue || j + r * NR < a.n_other) d[r * NR] = v[r];
+            } else {
+                d += (long long)j * a.out_stride;
+                const long long step = (long long)NR * a.out_stride;
+#pragma unroll
+                for (int r = 0; r < R; ++r, d += step) *d = v[r];
+            }
+        } else if constexpr (K::OP == OP_C2R_4A) {
+            const int col = sk_c2r4a_col<K>(a, c.i0, c.cnt, q);
+            if (col < 0) return;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int k = j + r * NR;
+                float2 x = c_tw<K::SIGN>(v[r], cross_tw(a, 2LL * col * k));
+                if (a.flags & TF_SCALE) x = c_scale(x, a.scale);
+                static_cast<float2*>(a.dst)[c.out_base - c.i0 + col + (long long)k * a.out_stride] = x;
+            }
+        } else if constexpr (K::OP == OP_C2R_HALF) {  // the factor 2 is in pass 0
+            float2* d = static_cast<float2*>(a.dst) + c.out_base + (long long)q * a.out_idist + j;
+#pragma unroll
+            for (int r = 0; r < R; ++r) d[r * NR] = v[r];
+        } else if constexpr (K::OP == OP_C2R_PAIR) {
+            const int row = 2 * (c.i0 + q);
+            float* d = static_cast<float*>(a.dst) + (long long)row * a.out_idist + j;
+#pragma unroll
+            for (int r = 0; r < R; ++r) d[r * NR] = v[r].x;
+            if (row + 1 < a.rows) {
+                d += a.out_idist;
+#pragma unroll
+                for (int r = 0; r < R; ++r) d[r * NR] = v[r].y;
             }
         }
+    }
+
+    SIP_HD static void write_global(int tid, const TileArgs& a, const TileCtx& c, Regs& rg) {
+        static_assert(LAST, "global store from the last pass only");
+#pragma unroll
+        for (int s = 0; s < S; ++s) store_slot(tid, s, a, c, rg.v[s]);
     }
 };
 
@@ -805,6 +920,28 @@ SIP_HD void sk_post(int tid, const TileArgs& a, const TileCtx& c, const float2* 
 // real twiddles W_{2M}^{u + r NR} = W_{2M}^u W_{2R}^r need table entries of
 // u only, times compile-time constants.
 
+// X[k] (into A[r]) and X[M - k] (into B[R - 1 - r]) from Z[k] = A[r], Z[M - k] =
+// B[R - 1 - r], with w2 = W_{2M}^{k0} / 2 for k = k0 + r M/R: X[k] = (E + W O) / 2,
+// X[M - k] = conj(E - W O) / 2, the halves folded into the twiddle and the sums.
+template <int R, int r>
+SIP_HD void sk_r2c_bins(float2 w2, float2 (&A)[R], float2 (&B)[R]) {
+    const float2 z = A[r], zm = B[R - 1 - r];
+    const float2 e = make_float2(z.x + zm.x, z.y - zm.y);
+    const float2 o = make_float2(z.y + zm.y, zm.x - z.x);
+    const float2 t = c_mul(tw_const<2 * R, r, -1>(w2), o);
+    A[r] = make_float2(0.5f * e.x + t.x, 0.5f * e.y + t.y);
+    B[R - 1 - r] = make_float2(0.5f * e.x - t.x, t.y - 0.5f * e.y);
+}
+
+template <int R>
+SIP_HD void sk_conj_all(float2 (&A)[R], float2 (&B)[R]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        A[r].y = -A[r].y;
+        B[r].y = -B[r].y;
+    }
+}
+
 // Last pass of an R2C_HALF tile, post-process fused, output to global memory.
 template <class K>
 SIP_HD void sk_pair_last_r2c(int tid, const TileArgs& a, const TileCtx& c, const float2* buf) {
@@ -817,7 +954,6 @@ SIP_HD void sk_pair_last_r2c(int tid, const TileArgs& a, const TileCtx& c, const
     constexpr int S = (TOTAL + K::T - 1) / K::T;
     static_assert(K::span(PASS) == NR, "the last pass spans N / R");
     const bool cj = (a.flags & TF_CONJ_OUT) != 0;
-    const bool sc = (a.flags & TF_SCALE) != 0;
     float2* dst = static_cast<float2*>(a.dst);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
@@ -847,29 +983,27 @@ SIP_HD void sk_pair_last_r2c(int tid, const TileArgs& a, const TileCtx& c, const
                 });
         }
         dft<R, K::SIGN>(A);
-        if (mirror) dft<R, K::SIGN>(B);
-        const float2 w2u = sk_tw2<K>(a, c, u);
-        float2* out = dst + c.out_base + (long long)q * a.out_idist;
-        sk_static_for<0, R>([&](auto ic) {
-            constexpr int r = decltype(ic)::value;
-            const int k = u + r * NR;
-            const float2 z = A[r];
-            const float2 zm = mirror ? B[R - 1 - r] : (u == 0 ? A[(R - r) % R] : A[R - 1 - r]);
-            const float2 w2 = tw_const<2 * R, r, -1>(w2u);  // W_{2M}^k
-            const float2 ev = make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
-            const float2 od = make_float2(0.5f * (z.y + zm.y), -0.5f * (z.x - zm.x));
-            const float2 t = c_mul(w2, od);
-            float2 x = c_add(ev, t);
-            float2 y = make_float2(ev.x - t.x, t.y - ev.y);  // X[M - k]
-            if (sc) {
-                x = c_scale(x, a.scale);
-                y = c_scale(y, a.scale);
-            }
-            out[k] = maybe_conj(x, cj);
-            // X[M - k] belongs to this thread when the mirror is another
-            // butterfly; for u = 0 only X[M] (r = 0) is not stored as some X[k]
-            if (mirror || (u == 0 && r == 0)) out[M - k] = maybe_conj(y, cj);
-        });
+        if (mirror) {
+            dft<R, K::SIGN>(B);
+        } else {  // the partners are this butterfly's own elements
+#pragma unroll
+            for (int r = 0; r < R; ++r) B[R - 1 - r] = u == 0 ? A[(R - r) % R] : A[R - 1 - r];
+        }
+        const float2 w2u = c_scale(sk_tw2<K>(a, c, u), 0.5f);
+        sk_static_for<0, R>([&](auto ic) { sk_r2c_bins<R, decltype(ic)::value>(w2u, A, B); });
+        if (cj) sk_conj_all(A, B);
+        float2* out = dst + c.out_base + (long long)q * a.out_idist + u;
+#pragma unroll
+        for (int r = 0; r < R; ++r) out[r * NR] = A[r];
+        out += M - 2 * u;
+        // X[M - k] belongs to this thread when the mirror is another
+        // butterfly; for u = 0 only X[M] (r = 0) is not stored as some X[k]
+        if (mirror) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) out[-r * NR] = B[R - 1 - r];
+        } else if (u == 0) {
+            out[0] = B[R - 1];
+        }
     }
 }
 
@@ -900,7 +1034,6 @@ SIP_HD void sk_pair_last_r2c_4b(int tid, const TileArgs& a, const TileCtx& c, co
     const int N1 = a.n_other;
     const long long M = (long long)N1 * N2;
     const bool cj = (a.flags & TF_CONJ_OUT) != 0;
-    const bool sc = (a.flags & TF_SCALE) != 0;
     float2* x = static_cast<float2*>(a.dst) + (c.out_base - c.i0);
 #pragma unroll
     for (int s = 0; s < S; ++s) {
@@ -933,26 +1066,24 @@ SIP_HD void sk_pair_last_r2c_4b(int tid, const TileArgs& a, const TileCtx& c, co
             for (int r = 1; r < R; ++r) B[r] = c_tw<K::SIGN>(B[r], w[r]);
         }
         dft<R, K::SIGN>(B);
-        const float2 w0 = cross_tw(a, k1 + (long long)N1 * j);  // W_{2M}^{k1 + N1 j}
-        sk_static_for<0, R>([&](auto ic) {
-            constexpr int r = decltype(ic)::value;
-            const long long kk = k1 + (long long)N1 * (j + r * NR);
-            const float2 z = A[r];
-            const float2 zm = (row0 && j == 0) ? A[(R - r) % R] : B[R - 1 - r];
-            const float2 w2 = tw_const<2 * R, r, -1>(w0);  // W_{2M}^{kk}
-            const float2 ev = make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
-            const float2 od = make_float2(0.5f * (z.y + zm.y), -0.5f * (z.x - zm.x));
-            const float2 t = c_mul(w2, od);
-            float2 xk = c_add(ev, t);
-            float2 xm = make_float2(ev.x - t.x, t.y - ev.y);  // X[M - kk]; X[M] for kk = 0
-            if (sc) {
-                xk = c_scale(xk, a.scale);
-                xm = c_scale(xm, a.scale);
-            }
-            x[kk] = maybe_conj(xk, cj);
-            if (!self) x[M - kk] = maybe_conj(xm, cj);
-            if (row0 && j == 0 && r == 0) x[M] = maybe_conj(xm, cj);
-        });
+        if (row0 && j == 0) {  // butterfly 0 is its own mirror: element r pairs with R - r
+#pragma unroll
+            for (int r = 0; r < R; ++r) B[R - 1 - r] = A[(R - r) % R];
+        }
+        const float2 w0 = c_scale(cross_tw(a, k1 + (long long)N1 * j), 0.5f);  // W_{2M}^{k1 + N1 j} / 2
+        sk_static_for<0, R>([&](auto ic) { sk_r2c_bins<R, decltype(ic)::value>(w0, A, B); });
+        if (cj) sk_conj_all(A, B);
+        const long long step = (long long)N1 * NR;
+        float2* xk = x + k1 + (long long)N1 * j;
+        float2* xm = x + (M - k1 - (long long)N1 * j);
+#pragma unroll
+        for (int r = 0; r < R; ++r, xk += step) *xk = A[r];
+        if (!self) {
+#pragma unroll
+            for (int r = 0; r < R; ++r, xm -= step) *xm = B[R - 1 - r];
+        } else if (row0 && j == 0) {
+            *xm = B[R - 1];  // X[M]
+        }
     }
 }
 
@@ -970,10 +1101,12 @@ struct SkPairFirstC2R {
         float2 a[S][R], b[S][R];
     };
 
-    // Z[n], Z[M - n] from x = X[n], y = X[M - n] and w = W_{2M}^n.
-    SIP_HD static void prep(float2 x, float2 y, float2 w, float2& zn, float2& zm) {
-        const float2 e = make_float2(0.5f * (x.x + y.x), 0.5f * (x.y - y.y));
-        const float2 d = make_float2(0.5f * (x.x - y.x), 0.5f * (x.y + y.y));
+    // 2 Z[n], 2 Z[M - n] from x = X[n], y = X[M - n] (conjugated for
+    // sg = -1) and w = W_{2M}^n; the output's factor 2 is this one.
+    SIP_HD static void prep(float2 x, float2 y, float sg, float2 w, float2& zn, float2& zm) {
+        const float yy = sg * y.y;
+        const float2 e = make_float2(x.x + y.x, sg * x.y - yy);
+        const float2 d = make_float2(x.x - y.x, sg * x.y + yy);
         const float2 od = c_mulc(d, w);
         zn = make_float2(e.x - od.y, e.y + od.x);
         zm = make_float2(e.x + od.y, od.x - e.y);
@@ -983,7 +1116,7 @@ struct SkPairFirstC2R {
     // pre-processed and transformed; false when the slot has no unit.
     SIP_HD static bool read_slot(int tid, int s, const TileArgs& a, const TileCtx& c, const float2* stage,
                                  float2 (&A)[R], float2 (&B)[R]) {
-        const bool cj = (a.flags & TF_CONJ_IN) != 0;
+        const float sg = (a.flags & TF_CONJ_IN) != 0 ? -1.f : 1.f;
         const int f = tid + s * K::T;
         if (TOTAL % K::T != 0 && f >= TOTAL) return false;
         const int q = f / U;
@@ -1001,12 +1134,12 @@ struct SkPairFirstC2R {
         sk_static_for<0, R>([&](auto ic) {
             constexpr int r = decltype(ic)::value;
             const int n = u + r * NR;
-            float2 x = maybe_conj(row[n], cj), y = maybe_conj(row[M - n], cj);
-            if (n == 0) {
+            float2 x = row[n], y = row[M - n];
+            if (r == 0 && n == 0) {
                 x.y = 0.f;
                 y.y = 0.f;
             }
-            prep(x, y, tw_const<2 * R, r, -1>(wu), A[r], B[R - 1 - r]);
+            prep(x, y, sg, tw_const<2 * R, r, -1>(wu), A[r], B[R - 1 - r]);
         });
         if (mirror) dft<R, K::SIGN>(B);
         dft<R, K::SIGN>(A);
@@ -1056,7 +1189,6 @@ SIP_HD void sk_pair_last_r2c_rows(int tid, const TileArgs& a, const TileCtx& c, 
     constexpr int S = (TOTAL + K::T - 1) / K::T;
     static_assert(N % 2 == 1 && K::span(PASS) == NR, "odd lengths; the last pass spans N / R");
     const bool cj = (a.flags & TF_CONJ_OUT) != 0;
-    const bool sc = (a.flags & TF_SCALE) != 0;
     float2* dst = static_cast<float2*>(a.dst);
     const int r0 = 2 * c.i0;
     const int nrows = (a.rows - r0) < 2 * c.cnt ? (a.rows - r0) : 2 * c.cnt;
@@ -1086,30 +1218,41 @@ SIP_HD void sk_pair_last_r2c_rows(int tid, const TileArgs& a, const TileCtx& c, 
             dft<R, K::SIGN>(B);
         }
         dft<R, K::SIGN>(A);
+        // element r of butterfly u is bin u + r NR, below N/2 for 2 r < R
+        // (2 u < NR); the others' bins are the mirror's elements R - 1 - r
         const long long ra = r0 + 2 * q;
         float2* outa = dst + ra * a.out_idist;
-        float2* outb = outa + a.out_idist;
         const bool second = 2 * q + 1 < nrows;
-        auto store = [&](int b, float2 z, float2 zm) {
-            float2 xa = make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
-            float2 xb = make_float2(0.5f * (z.y + zm.y), -0.5f * (z.x - zm.x));
-            if (sc) {
-                xa = c_scale(xa, a.scale);
-                xb = c_scale(xb, a.scale);
+        if (mirror) {
+            float2 xa[R], xb[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float2 z = 2 * r < R ? A[r] : B[R - 1 - r], zm = 2 * r < R ? B[R - 1 - r] : A[r];
+                xa[r] = make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
+                xb[r] = make_float2(0.5f * (z.y + zm.y), -0.5f * (z.x - zm.x));
             }
-            outa[b] = maybe_conj(xa, cj);
-            if (second) outb[b] = maybe_conj(xb, cj);
-        };
-        sk_static_for<0, R>([&](auto ic) {
-            constexpr int r = decltype(ic)::value;
-            if (mirror) {
-                const int k = u + r * NR;
-                if (2 * k < N) store(k, A[r], B[R - 1 - r]);
-                else store(N - k, B[R - 1 - r], A[r]);
-            } else if constexpr (2 * r * NR < N) {
-                store(r * NR, A[r], A[(R - r) % R]);
+            if (cj) sk_conj_all(xa, xb);
+            float2* lo = outa + u;
+            float2* hi = outa + (N - u);
+#pragma unroll
+            for (int r = 0; r < R; ++r) *(2 * r < R ? lo + r * NR : hi - r * NR) = xa[r];
+            if (second) {
+                lo += a.out_idist;
+                hi += a.out_idist;
+#pragma unroll
+                for (int r = 0; r < R; ++r) *(2 * r < R ? lo + r * NR : hi - r * NR) = xb[r];
             }
-        });
+        } else {
+            float2* outb = outa + a.out_idist;
+#pragma unroll
+            for (int r = 0; 2 * r < R; ++r) {
+                const float2 z = A[r], zm = A[(R - r) % R];
+                float2 xa = make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
+                float2 xb = make_float2(0.5f * (z.y + zm.y), -0.5f * (z.x - zm.x));
+                outa[r * NR] = maybe_conj(xa, cj);
+                if (second) outb[r * NR] = maybe_conj(xb, cj);
+            }
+        }
     }
 }
 
@@ -1304,6 +1447,7 @@ struct SkPick<false, T, F> {
 // between reading and writing, so only one slot's values are live).
 template <class K>
 SIP_HD void sk_pass0_split(int tid, const TileArgs& a, const TileCtx& c, const float2* stage, float2* work) {
+    stage += sk_stage_shift<K>(a, c);
     if constexpr (K::MPAIR && (K::OP == OP_C2R_HALF || K::OP == OP_C2R_PAIR)) {
         using PP = typename SkPick<K::OP == OP_C2R_HALF, SkPairFirstC2R<K>, SkPairFirstC2RRows<K>>::type;
 #pragma unroll
