@@ -20,6 +20,7 @@
 #include <new>
 #include <sstream>
 #include <thread>
+#include <tuple>
 #include <condition_variable>
 #include <chrono>
 #include <set>
@@ -130,6 +131,41 @@ std::vector<int> jit_radices(int n) {
     if (r.first >= 1e29 || r.second.size() > (size_t)kMaxPasses) return {};
     std::sort(r.second.begin(), r.second.end(), std::greater<int>());
     return r.second;
+}
+
+// Radices of a pulse tile, the last one first of all small: its pass holds a
+// butterfly's values and as many filter values (sk_kernel.cuh sk_ip_turn), and
+// with 128 registers a thread it spills from about 20 up.  2^9 27 as 27 x 32 x
+// 16 runs 2427 rows in 234 us, as 24 x 24 x 24 (164 bytes spilled) in 272 us.
+std::vector<int> jit_pulse_radices(int n) {
+    std::vector<int> best;
+    double cost = 1e30;
+    for (int last = 18; last >= 2; --last) {
+        if (n % last != 0) continue;
+        std::vector<int> r = jit_radices(n / last);
+        if (r.empty() && n != last) continue;
+        r.push_back(last);
+        double c = last > 16 ? 0.01 : 0.0;
+        for (int x : r) c += jit_radix_cost(x);
+        if (c < cost && r.size() <= (size_t)kMaxPasses) {
+            cost = c;
+            best = r;
+        }
+    }
+    return best.empty() ? jit_radices(n) : best;
+}
+
+// sk_ip_layout, searched once per radix order, tile and mode.
+SkIpLayout ip_layout(const std::vector<int>& radices, int P, int mode) {
+    static std::mutex& mu = *new std::mutex;
+    static auto& known = *new std::map<std::tuple<std::vector<int>, int, int>, SkIpLayout>;
+    const auto key = std::make_tuple(radices, P, mode);
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(key);
+    if (it == known.end())
+        it = known.emplace(key, sk_ip_layout(radices.data(), (int)radices.size(), P, mode == SK_COLS,
+                                             mode == SK_ROWS_T)).first;
+    return it->second;
 }
 
 // Threads so that no pass holds more than `e` values per thread (one
@@ -260,7 +296,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     c.sign = sign;
     c.tw4 = tw4;
     c.n = n;
-    c.radices = order != nullptr ? *order : jit_radices(n);
+    c.radices = order != nullptr ? *order : op == OP_PC ? jit_pulse_radices(n) : jit_radices(n);
     // Tuning overrides (sweeps; unset in normal use): SIP_FFT_JIT_RADICES
     // ("25,15,8", must multiply to n), SIP_FFT_JIT_P, SIP_FFT_JIT_T,
     // SIP_FFT_JIT_MINB, SIP_FFT_JIT_STAGES, SIP_FFT_JIT_TWB (the SK_TW_* bits
@@ -313,24 +349,53 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     // the basis table through L1 over run-time compiled C2C rows of 544 to
     // 8160 points.  Mirrored butterfly pairs (on request) apply to real
     // half-length tiles of two or more passes.
-    c.twb = ovr_int("SIP_FFT_JIT_TWB", SK_TW_BASIS | SK_TW_SMEM | SK_SPLIT_PASS0);
-    if (c.twb < 0 || c.twb > 15) return false;
+    c.twb = ovr_int("SIP_FFT_JIT_TWB", op == OP_PC ? SK_TW_BASIS | SK_IN_PLACE
+                                                   : SK_TW_BASIS | SK_TW_SMEM | SK_SPLIT_PASS0);
+    if (c.twb < 0 || c.twb > 31) return false;
     if ((c.twb & SK_MIRROR_PAIR) && (!real_op || c.radices.size() < 2)) c.twb &= ~SK_MIRROR_PAIR;
-    if ((c.twb & SK_SPLIT_PASS0) && (c.radices.size() < 2 || op == OP_PC)) c.twb &= ~SK_SPLIT_PASS0;
-    const long long buf = (long long)sk_buffer_values(op, c.P, n, r0, c.twb) * 8;
-    long long tws = (long long)sk_tws_values(op, n, c.radices.data(), (int)c.radices.size(), c.twb) * 8;
+    if ((c.twb & SK_SPLIT_PASS0) && (c.radices.size() < 2 || (op == OP_PC && !(c.twb & SK_IN_PLACE))))
+        c.twb &= ~SK_SPLIT_PASS0;
+    if (c.radices.size() < 2) c.twb &= ~SK_IN_PLACE;
+    const bool inplace = (c.twb & SK_IN_PLACE) != 0;
+    if (inplace && (op == OP_R2C_HALF || op == OP_R2C_PAIR)) c.twb |= SK_MIRROR_PAIR;
+    SkIpLayout lay{0, 0};
+    if (inplace) {
+        lay = ip_layout(c.radices, c.P, mode);
+        c.LD = lay.ld;
+    }
+    const long long buf =
+        8LL * (inplace ? sk_ip_buffer_values(c.P, lay) : sk_buffer_values(op, c.P, n, r0, c.twb));
+    const long long staged = 8LL * ((sk_stage_slots(op, c.P, n, c.twb) + 1) / 2 * 2);  // in-place tiles' input
+    long long tws = 8LL * sk_tws_values(op, n, c.radices.data(), (int)c.radices.size(), c.twb);
     if (buf + tws > kMaxTileSmem && (c.twb & SK_TW_SMEM)) {  // no room for the staged twiddles
         c.twb &= ~SK_TW_SMEM;
         tws = 0;
     }
-    if (2 * buf + tws <= kMaxTileSmem) c.stages = 2;
+    const long long both = inplace ? buf + ((c.twb & SK_SPLIT_PASS0) ? staged : 0) : 2 * buf;
+    if (inplace && (!(c.twb & SK_SPLIT_PASS0) || both + tws > kMaxTileSmem)) c.stages = 1;
+    else if (both + tws <= kMaxTileSmem) c.stages = 2;
     else if (buf + tws <= kMaxTileSmem) c.stages = 1;
     else return false;
     if (ovr_int("SIP_FFT_JIT_STAGES", 0) == 1) c.stages = 1;
     if (c.stages != 2) c.twb &= ~SK_SPLIT_PASS0;  // a split pass 0 uses the second buffer as its work layout
-    c.smem = (int)(c.stages * buf + tws);
+    if (inplace && buf + tws > kMaxTileSmem) return false;
+    c.smem = (int)((c.stages == 2 ? both : buf) + tws);
     const int smem_ctas = std::max<int>(1, (228 * 1024) / (c.smem + 1024));
     c.minb = std::max(1, std::min(65536 / (T * 128), smem_ctas));
+    if (inplace && op == OP_PC) {
+        // A pulse tile runs in place, where a thread holds one butterfly at a
+        // time whatever the tile's size, so the threads are chosen for the
+        // residency: 16 warps per SM at 128 registers, in CTAs as small as the
+        // shared memory allows (a CTA waits at each of its barriers, the others
+        // go on).  Rows of 4320, 33.5 M values: 229 us with 4 CTAs of 128
+        // threads, 251 with 2 of 256, 328 with 1 of 288; 8640: 248 us with 2 of
+        // 256, 326 with 1 of 384.  `values` other than 32: half the CTAs, for
+        // tiles that spill.
+        const int fit = std::max<int>(1, (228 * 1024) / ((int)(buf + tws) + 1024));
+        c.T = fit >= 4 ? 128 : fit >= 2 ? 256 : 512;
+        c.minb = std::max(1, std::min(fit, 512 / c.T) / (per_thread == 32 ? 1 : 2));
+        if (ovr_int("SIP_FFT_JIT_T", 0) > 0) c.T = ovr_int("SIP_FFT_JIT_T", 0);
+    }
     if (ovr_int("SIP_FFT_JIT_MINB", 0) > 0) c.minb = ovr_int("SIP_FFT_JIT_MINB", 0);
     *out = c;
     return true;
@@ -497,7 +562,7 @@ std::vector<JitCfg> jit_candidates(int op, int mode, int sign, bool tw4, int n, 
     // fits in the registers without spills varies (a pulse tile of 4320
     // points as 18 x 16 x 15 on 288 threads spills 240 bytes per thread,
     // as 15 x 16 x 18 none)
-    std::vector<std::vector<int>> orders = {jit_radices(n)};
+    std::vector<std::vector<int>> orders = {op == OP_PC ? jit_pulse_radices(n) : jit_radices(n)};
     if (!orders[0].empty() && orders[0].front() != orders[0].back())
         orders.push_back(std::vector<int>(orders[0].rbegin(), orders[0].rend()));
     for (size_t oi = 0; oi < orders.size(); ++oi)
@@ -511,7 +576,7 @@ std::vector<JitCfg> jit_candidates(int op, int mode, int sign, bool tw4, int n, 
         // thread, one of 8 warps 255.  So each candidate is also tried with
         // its threads rounded down to a multiple of 128 (more values per
         // thread) and the register target left to the compiler.
-        if (c.T % 128 != 0 && c.T > 128) {
+        if (c.T % 128 != 0 && c.T > 128 && op != OP_PC) {
             JitCfg r = c;
             r.T = c.T / 128 * 128;
             bool ok = true;

@@ -36,8 +36,86 @@ SIP_HD constexpr int sk_index(int n, int r0) { return r0 % 2 == 0 ? n + n / sk_p
 SIP_HD constexpr int sk_pitch(int n, int r0) {
     return ((sk_index(n - 1, r0) + 1) & 1) ? sk_index(n - 1, r0) + 1 : sk_index(n - 1, r0) + 2;
 }
-// The TWB bits (SK_TW_BASIS, SK_TW_SMEM, SK_MIRROR_PAIR, SK_SPLIT_PASS0) are
-// defined in sk_modes.h.
+// The TWB bits (SK_TW_BASIS, SK_TW_SMEM, SK_MIRROR_PAIR, SK_SPLIT_PASS0,
+// SK_IN_PLACE) are defined in sk_modes.h.
+
+// In-place layout (SK_IN_PLACE): the element with mixed-radix digits
+// d_0 .. d_{m-1} (n = d_0 N/R_0 + d_1 N/(R_0 R_1) + ...) of transform q lives at
+// slot sum d_i S_i of the transform: S_i = N/(R_0..R_i) for i > 0, and S_0 and the
+// pitch of the transforms padded by up to 15 slots.  Row tiles keep
+// transform q at q * pitch, column tiles interleave their P transforms
+// (slot * P + q).
+//
+// The pads are chosen by counting: of the 16 candidates, the one whose passes
+// need the fewest shared-memory wavefronts (a wavefront serves 16 lanes in
+// 16 different 8-byte banks; lane order as in SkPass::butterfly_index).
+struct SkIpLayout {
+    int s0, ld;
+};
+SIP_HD constexpr int sk_ip_inner(const int* rs, int np, int i) {  // N / (R_0 .. R_i)
+    int s = 1;
+    for (int p = np - 1; p > i; --p) s *= rs[p];
+    return s;
+}
+// Slot of butterfly j of pass p.
+SIP_HD constexpr int sk_ip_slot_of(const int* rs, int np, int p, int s0, int j) {
+    int l = 1;
+    for (int i = 0; i < p; ++i) l *= rs[i];
+    const int m_count = sk_ip_inner(rs, np, p);
+    int k = p == np - 1 ? j : j / m_count, m = p == np - 1 ? 0 : j % m_count, s = 0;
+    for (int i = 0; i < p; ++i) {
+        s += (k % rs[i]) * (i == 0 ? s0 : sk_ip_inner(rs, np, i));
+        k /= rs[i];
+    }
+    return s + m;
+}
+SIP_HD constexpr int sk_ip_wavefronts(const int* rs, int np, int P, bool cols, bool cols_last, int s0, int ld) {
+    int n = 1, total = 0;
+    for (int i = 0; i < np; ++i) n *= rs[i];
+    for (int p = 0; p < np; ++p) {
+        const int nr = n / rs[p];
+        const bool q_first = cols || (cols_last && p == np - 1);
+        for (int h = 0; h < 6; ++h) {
+            int hit[16] = {}, worst = 0;
+            for (int lane = 0; lane < 16; ++lane) {
+                const int b = h * 16 + lane;
+                if (b >= P * nr) break;
+                const int q = q_first ? b % P : b / nr, j = q_first ? b / P : b % nr;
+                const int slot = sk_ip_slot_of(rs, np, p, s0, j);
+                const int bank = (cols ? slot * P + q : q * ld + slot) % 16;
+                if (++hit[bank] > worst) worst = hit[bank];
+            }
+            total += worst;
+        }
+    }
+    return total;
+}
+SIP_HD constexpr SkIpLayout sk_ip_layout(const int* rs, int np, int P, bool cols, bool cols_last) {
+    const int base = sk_ip_inner(rs, np, 0);
+    SkIpLayout best{base, rs[0] * base};
+    int cost = 1 << 30;
+    for (int pad = 0; pad < 16; ++pad) {
+        const int c = sk_ip_wavefronts(rs, np, 1, cols, false, base + pad, 0) +
+                      (cols ? sk_ip_wavefronts(rs, np, P, true, false, base + pad, 0) : 0);
+        if (c < cost) {
+            cost = c;
+            best.s0 = base + pad;
+        }
+    }
+    const int row = rs[0] * best.s0;
+    best.ld = row;
+    if (cols || P == 1) return best;
+    cost = 1 << 30;
+    for (int pad = 0; pad < 16; ++pad) {
+        const int c = sk_ip_wavefronts(rs, np, P, false, cols_last, best.s0, row + pad);
+        if (c < cost) {
+            cost = c;
+            best.ld = row + pad;
+        }
+    }
+    return best;
+}
+SIP_HD constexpr int sk_ip_buffer_values(int p, SkIpLayout lay) { return (p * lay.ld + 1) / 2 * 2; }
 
 SIP_HD constexpr int sk_twcount(int r, bool basis) { return basis ? basis_count(r) : r - 1; }
 // Entries per table row of pass p in shared memory: all L values k of the
@@ -112,6 +190,7 @@ struct SkCfg {
     static constexpr bool TWS = (TWB_ & SK_TW_SMEM) != 0;
     static constexpr bool MPAIR = (TWB_ & SK_MIRROR_PAIR) != 0;
     static constexpr bool SPLIT = (TWB_ & SK_SPLIT_PASS0) != 0;
+    static constexpr bool INPLACE = (TWB_ & SK_IN_PLACE) != 0;
     // The configuration's own operation (SkView below re-labels OP for the
     // halves of a pulse tile; the staged twiddle layout follows CFG_OP).
     static constexpr int CFG_OP = OP_;
@@ -135,8 +214,39 @@ struct SkCfg {
 
     static constexpr int rad_list[] = {Rs...};
     static constexpr int STAGE = sk_stage_values(OP, P, N);
-    static constexpr int LD = sk_pitch(N, radix(0));
-    static constexpr int BUF = sk_buffer_values(OP, P, N, radix(0), FLAGS);
+    // In-place layout (sk_ip_layout).  DIRECT: pass 0 reads global memory and
+    // the work layout is the only buffer; else the input is staged.
+    static constexpr bool DIRECT = INPLACE && !SPLIT;
+    static constexpr SkIpLayout LAY = INPLACE ? sk_ip_layout(rad_list, NP, P, MODE == SK_COLS, MODE == SK_ROWS_T)
+                                              : SkIpLayout{0, 0};
+    static constexpr int LD = INPLACE ? LAY.ld : sk_pitch(N, radix(0));
+    static constexpr int BUF = INPLACE ? sk_ip_buffer_values(P, LAY) : sk_buffer_values(OP, P, N, radix(0), FLAGS);
+    static constexpr bool INTERLEAVED = INPLACE && MODE == SK_COLS;
+    SIP_HD static constexpr int ip_at(int q, int s) { return INTERLEAVED ? s * P + q : q * LD + s; }
+    static constexpr int ip_stride(int p) { return p == 0 ? LAY.s0 : sk_ip_inner(rad_list, NP, p); }
+    static constexpr int ip_step(int p) { return ip_stride(p) * (INTERLEAVED ? P : 1); }
+    // Slot of the digits before pass p, whose transformed values count k < span(p).
+    template <int PASS_>
+    SIP_HD static constexpr int ip_low(int k) {
+        int s = 0, l = 1;
+#pragma unroll
+        for (int i = 0; i < PASS_; ++i) {
+            const int r = radix(i);
+            s += (i + 1 < PASS_ ? (k / l) % r : k / l) * ip_stride(i);
+            l *= r;
+        }
+        return s;
+    }
+    // Slots of element r of butterfly u: the last pass's input, pass 0's output
+    // (row tiles).
+    SIP_HD static constexpr int last_slot(int u, int r) {
+        if constexpr (INPLACE) return ip_low<NP - 1>(u) + r;
+        else return idx(u + r * (N / radix(NP - 1)));
+    }
+    SIP_HD static constexpr int first_slot(int u, int r) {
+        if constexpr (INPLACE) return u + r * ip_step(0);
+        else return idx(u * radix(0) + r);
+    }
     // Staged twiddles (SK_TW_SMEM): per pass p with span > 1, twcount rows
     // of tws_stride(p) entries from tws_off(p), then TW2S real twiddles.
     static constexpr int tws_stride(int p) { return sk_tws_stride(CFG_OP, FLAGS, p, NP, span(p)); }
@@ -149,7 +259,11 @@ struct SkCfg {
     static constexpr int TW2_OFF = tws_off(NP);
     static constexpr int TW2S = sk_tw2s(CFG_OP, N, radix(0), radix(NP - 1), FLAGS);
     static constexpr int TWSM = TWS ? (TW2_OFF + TW2S + 1) / 2 * 2 : 0;
-    static constexpr int SMEM = 2 * BUF * 8 + TWSM * 8;
+    // Dynamic shared memory (bytes) of the kernel with STAGES buffers.
+    static constexpr int smem_bytes(int stages) {
+        return 8 * ((INPLACE ? BUF + (SPLIT ? (sk_stage_slots(OP, P, N, FLAGS) + 1) / 2 * 2 : 0) : stages * BUF) +
+                    TWSM);
+    }
     // CTAs per SM the shared memory allows with two stages (228 KB per SM,
     // 1 KB reserved per CTA); used as the register-allocation target.
     static constexpr int smem_ctas(int stages) {
@@ -175,7 +289,8 @@ struct SkCfg {
                   "R2C tiles run the forward transform");
     static_assert(!MPAIR || (OP != OP_C2R_HALF && OP != OP_C2R_PAIR) || SIGN > 0,
                   "C2R tiles run the inverse transform");
-    static_assert(!SPLIT || (NP >= 2 && OP != OP_PC), "a split pass 0 needs a later pass, and no pulse tile");
+    static_assert(!SPLIT || (NP >= 2 && (OP != OP_PC || INPLACE)), "a split pass 0 needs a later pass, and no pulse tile");
+    static_assert(!INPLACE || (NP >= 2 && OP != OP_C2R_4A && OP != OP_R2C_4B), "in-place tiles: two or more passes");
     static_assert(TWSM == sk_tws_values(OP_, N_, rad_list, NP, TWB_), "staged twiddle layout");
 };
 
@@ -571,9 +686,17 @@ SIP_HD float2 sk_c2r4a_input(const TileArgs& a, const TileCtx& c, const float2* 
 }
 
 // Value n of transform q as pass 0 reads it from the staged input.
+// Direct tiles pass the tile's input in global memory as `stage`: rows
+// have the same layout there, columns are in_stride apart.
 template <class K>
 SIP_HD float2 sk_input(const TileArgs& a, const TileCtx& c, const float2* stage, int q, int n) {
     constexpr int N = K::N;
+    if constexpr (K::DIRECT && K::OP == OP_C2C && K::MODE == SK_COLS) return stage[q + n * a.in_stride];
+    if constexpr (K::DIRECT && K::OP == OP_R2C_PAIR) {
+        const float* s = reinterpret_cast<const float*>(stage);
+        const bool second = 2 * (c.i0 + q) + 1 < a.rows;  // an odd batch's last row has no partner
+        return make_float2(s[(2 * q) * N + n], second ? s[(2 * q + 1) * N + n] : 0.f);
+    }
     if constexpr (K::OP == OP_PC) {
         if (a.flags & TF_BLUE) {  // Bluestein: chirp times the input, zero padded
             const int nb = a.n_other;
@@ -594,7 +717,8 @@ SIP_HD float2 sk_input(const TileArgs& a, const TileCtx& c, const float2* stage,
         constexpr int H = N / 2 + 1;
         const int kk = n <= N / 2 ? n : N - n;
         float2 xa = stage[(2 * q) * H + kk];
-        float2 xb = stage[(2 * q + 1) * H + kk];
+        const bool second = !K::DIRECT || 2 * (c.i0 + q) + 1 < a.rows;
+        float2 xb = second ? stage[(2 * q + 1) * H + kk] : make_float2(0.f, 0.f);
         if (kk == 0 || 2 * kk == N) {
             xa.y = 0.f;
             xb.y = 0.f;
@@ -632,6 +756,27 @@ struct SkPass {
     static constexpr bool COL = K::colmap(PASS);
     static constexpr bool LAST = PASS == K::NP - 1;
     using Regs = PassRegs<R, S>;
+    // Butterfly j of a pass has twiddle index k < L and element index m:
+    // j = m L + k, or k M + m in the middle passes of an in-place tile (lanes
+    // along m take adjacent slots).
+    static constexpr int M = NR / L;
+    SIP_HD static void split_index(int j, int& k, int& m) {
+        if (K::INPLACE && !LAST) {
+            k = j / M;
+            m = j % M;
+        } else {
+            k = j % L;
+            m = j / L;
+        }
+    }
+    // First slot of butterfly j of transform q (in-place layout; element r
+    // is ip_step(PASS) slots further).
+    SIP_HD static int ip_slot(int q, int j) {
+        int k, m;
+        split_index(j, k, m);
+        return K::ip_at(q, K::template ip_low<PASS>(k) + m);
+    }
+
     SIP_HD static void butterfly_index(int b, int& q, int& j) {
         if (COL) {
             q = b % K::P;
@@ -650,6 +795,13 @@ struct SkPass {
         if (TOTAL % K::T != 0 && b >= TOTAL) return false;
         int q, j;
         butterfly_index(b, q, j);
+        if constexpr (K::DIRECT && PASS == 0 && !K::WORK_IN) {
+            if (q >= c.cnt) {  // a partial tile: nothing to read, nothing is stored
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = make_float2(0.f, 0.f);
+                return true;
+            }
+        }
         if constexpr (PASS == 0 && !K::WORK_IN && K::OP == OP_C2R_HALF) {
             // C2R pre-process: the twiddle of element n = j + r NR is
             // W_{2M}^{j + r NR} = W_{2M}^j W_{2R}^r, one table entry per
@@ -669,6 +821,10 @@ struct SkPass {
                 const float2 od = c_mulc(d, tw_const<2 * R, r, -1>(wj));
                 v[r] = make_float2(e.x - od.y, e.y + od.x);
             });
+        } else if constexpr (K::INPLACE && (PASS > 0 || K::WORK_IN)) {
+            const float2* p = buf + ip_slot(q, j);
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[r] = p[r * K::ip_step(PASS)];
         } else {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -681,8 +837,10 @@ struct SkPass {
         if constexpr (L > 1) {
             // twiddle-major tables: consecutive k of a warp read consecutive
             // entries
+            int k, m;
+            split_index(j, k, m);
             float2 w[R];
-            sk_pass_twiddles<K, PASS>(a, c, j % L, w);
+            sk_pass_twiddles<K, PASS>(a, c, k, w);
 #pragma unroll
             for (int r = 1; r < R; ++r) v[r] = c_tw<K::SIGN>(v[r], w[r]);
         }
@@ -696,6 +854,12 @@ struct SkPass {
         if (TOTAL % K::T != 0 && b >= TOTAL) return;
         int q, j;
         butterfly_index(b, q, j);
+        if constexpr (K::INPLACE) {
+            float2* p = buf + ip_slot(q, j);
+#pragma unroll
+            for (int r = 0; r < R; ++r) p[r * K::ip_step(PASS)] = v[r];
+            return;
+        }
         const int o = (j / L) * L * R + j % L;
 #pragma unroll
         for (int r = 0; r < R; ++r) buf[q * K::LD + K::idx(o + r * L)] = v[r];
@@ -712,7 +876,8 @@ struct SkPass {
         for (int s = 0; s < S; ++s) write_slot(tid, s, buf, rg.v[s]);
     }
 
-    // Last pass straight to global memory: element k = j + r N/R of transform q.
+    // Last pass straight to global memory: element k = j + r N/R of transform q
+    // (a pulse tile's inverse half ends with pass 0 when it runs in place).
     // The flags are uniform branches around whole butterflies and the
     // addresses a base plus constant steps, so that a stored value costs its
     // store alone.
@@ -966,10 +1131,10 @@ SIP_HD void sk_pair_last_r2c(int tid, const TileArgs& a, const TileCtx& c, const
         const float2* row = buf + q * K::LD;
         float2 A[R], B[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) A[r] = row[K::idx(u + r * NR)];
+        for (int r = 0; r < R; ++r) A[r] = row[K::last_slot(u, r)];
         if (mirror) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) B[r] = row[K::idx(NR - u + r * NR)];
+            for (int r = 0; r < R; ++r) B[r] = row[K::last_slot(NR - u, r)];
         }
         if (u != 0) {
             float2 w[R];
@@ -1121,6 +1286,11 @@ struct SkPairFirstC2R {
         if (TOTAL % K::T != 0 && f >= TOTAL) return false;
         const int q = f / U;
         const int u = f - q * U;
+        if (K::DIRECT && q >= c.cnt) {  // a partial tile: nothing to read, nothing is stored
+#pragma unroll
+            for (int r = 0; r < R; ++r) A[r] = B[r] = make_float2(0.f, 0.f);
+            return true;
+        }
         const float2* row = stage + q * (M + 1);
         const float2 wu = sk_tw2<K>(a, c, u);
         // One code path for every unit: element r of butterfly u is Z[n] from
@@ -1154,10 +1324,10 @@ struct SkPairFirstC2R {
         const int u = f - q * U;
         float2* row = buf + q * K::LD;
 #pragma unroll
-        for (int r = 0; r < R; ++r) row[K::idx(u * R + r)] = A[r];
+        for (int r = 0; r < R; ++r) row[K::first_slot(u, r)] = A[r];
         if (u != 0 && 2 * u != NR) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) row[K::idx((NR - u) * R + r)] = B[r];
+            for (int r = 0; r < R; ++r) row[K::first_slot(NR - u, r)] = B[r];
         }
     }
 
@@ -1203,10 +1373,10 @@ SIP_HD void sk_pair_last_r2c_rows(int tid, const TileArgs& a, const TileCtx& c, 
         const float2* row = buf + q * K::LD;
         float2 A[R], B[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) A[r] = row[K::idx(u + r * NR)];
+        for (int r = 0; r < R; ++r) A[r] = row[K::last_slot(u, r)];
         if (mirror) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) B[r] = row[K::idx(NR - u + r * NR)];
+            for (int r = 0; r < R; ++r) B[r] = row[K::last_slot(NR - u, r)];
             float2 w[R];
             sk_pass_twiddles<K, PASS>(a, c, u, w);
 #pragma unroll
@@ -1367,8 +1537,8 @@ struct SkPairFirstC2RRows {
     static_assert(N % 2 == 1, "odd lengths");
 
     // Z[m] (lo) and Z[N - m] (hi) from bin m of both rows, m <= N/2.
-    SIP_HD static void bins(const float2* sa, const float2* sb, int m, bool fwd, float2& lo, float2& hi) {
-        float2 xa = sa[m], xb = sb[m];
+    SIP_HD static void bins(const float2* sa, const float2* sb, int m, bool second, bool fwd, float2& lo, float2& hi) {
+        float2 xa = sa[m], xb = second ? sb[m] : make_float2(0.f, 0.f);
         if (m == 0) {
             xa.y = 0.f;
             xb.y = 0.f;
@@ -1386,6 +1556,14 @@ struct SkPairFirstC2RRows {
         if (TOTAL % K::T != 0 && f >= TOTAL) return false;
         const int q = f / U;
         const int u = f - q * U;
+        if (K::DIRECT && q >= c.cnt) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) A[r] = B[r] = make_float2(0.f, 0.f);
+            return true;
+        }
+        // (a staged tile holds zeros for the missing partner of an odd
+        // batch's last row)
+        const bool second = !K::DIRECT || 2 * (c.i0 + q) + 1 < a.rows;
         const float2* sa = stage + (2 * q) * H;
         const float2* sb = sa + H;
         // one code path for every unit (u = 0 is its own mirror: B unused)
@@ -1394,7 +1572,7 @@ struct SkPairFirstC2RRows {
             const int n = u + r * NR;
             const bool low = 2 * n < N;
             float2 lo, hi;
-            bins(sa, sb, low ? n : N - n, fwd, lo, hi);
+            bins(sa, sb, low ? n : N - n, second, fwd, lo, hi);
             A[r] = low ? lo : hi;
             B[R - 1 - r] = low ? hi : lo;
         });
@@ -1410,10 +1588,10 @@ struct SkPairFirstC2RRows {
         const int u = f - q * U;
         float2* row = buf + q * K::LD;
 #pragma unroll
-        for (int r = 0; r < R; ++r) row[K::idx(u * R + r)] = A[r];
+        for (int r = 0; r < R; ++r) row[K::first_slot(u, r)] = A[r];
         if (u != 0) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) row[K::idx((NR - u) * R + r)] = B[r];
+            for (int r = 0; r < R; ++r) row[K::first_slot(NR - u, r)] = B[r];
         }
     }
 
@@ -1499,6 +1677,180 @@ SIP_HD void sk_mul(int tid, const TileArgs& a, const TileCtx& c, float2* buf) {
     }
 }
 
+// ------------------------------------------------------ in-place passes
+// SK_IN_PLACE.  The passes are those above (decimation in time, twiddles on
+// a pass's inputs); only the places differ: instead of the self-sorting
+// exchange, every pass writes its butterfly's outputs where its inputs
+// were, digit p of the time index becoming digit p of the frequency index.
+// Pass 0 reads global memory in natural order and the last pass, whose
+// lanes run along k, stores X[k + r N/R] in natural order, so nothing is ever
+// reordered.  A butterfly's slots belong to one thread within a pass: no
+// barrier between its reads and writes, one barrier per pass, one butterfly's
+// values live at a time, and one buffer instead of a staging and a work
+// buffer.  What hides the loads' latency is the number of resident CTAs.
+// Pulse tiles gain most: both halves of the self-sorting form need all of a
+// thread's values live across each exchange (240 to 700 spilled bytes from
+// 4320 points up, or one CTA per SM), the last pass, the filter product and
+// the first inverse pass three shared-memory round trips.  Rows of 4096, 8.4 M
+// values: 122 -> 52 us; Bluestein's c2c 6752 x 8192 (m = 13824): 3.25 -> 1.15 ms.
+
+// The tile's input in global memory: row tiles index it as their staged
+// image, column tiles by the column stride.
+template <class K>
+SIP_HD const float2* sk_ip_source(const TileArgs& a, const TileCtx& c) {
+    if constexpr (K::OP == OP_R2C_PAIR)
+        return reinterpret_cast<const float2*>(static_cast<const float*>(a.src) + 2LL * c.i0 * a.in_idist);
+    else if constexpr (K::OP == OP_C2R_PAIR)
+        return static_cast<const float2*>(a.src) + 2LL * c.i0 * a.in_idist;
+    else
+        return static_cast<const float2*>(a.src) + c.in_base;
+}
+
+// Pass 0 of the tile: its input `src` (global memory of a direct tile, else
+// the staging buffer) -> butterfly -> the work buffer.  `ready` runs
+// once, after the first slot's loads and before the first write (the barrier
+// behind which the previous tile's last pass has read its slots).
+template <class K, class Ready>
+SIP_HD void sk_ip_first(int tid, const TileArgs& a, const TileCtx& c, const float2* src, float2* buf, Ready&& ready) {
+    src += sk_stage_shift<K>(a, c);
+    if constexpr (K::MPAIR && (K::OP == OP_C2R_HALF || K::OP == OP_C2R_PAIR)) {
+        using PP = typename SkPick<K::OP == OP_C2R_HALF, SkPairFirstC2R<K>, SkPairFirstC2RRows<K>>::type;
+#pragma unroll
+        for (int s = 0; s < PP::S; ++s) {
+            float2 A[PP::R], B[PP::R];
+            const bool have = PP::read_slot(tid, s, a, c, src, A, B);
+            if (s == 0) ready();
+            if (have) PP::write_slot(tid, s, buf, A, B);
+        }
+    } else {
+        using SP = SkPass<K, 0>;
+#pragma unroll
+        for (int s = 0; s < SP::S; ++s) {
+            float2 v[SP::R];
+            const bool have = SP::read_slot(tid, s, a, c, src, v);
+            if (s == 0) ready();
+            if (have) SP::write_slot(tid, s, buf, v);
+        }
+    }
+}
+
+// A middle pass, in place.
+template <class K, int PASS>
+SIP_HD void sk_ip_middle(int tid, const TileArgs& a, const TileCtx& c, float2* buf) {
+    using SP = SkPass<K, PASS>;
+#pragma unroll
+    for (int s = 0; s < SP::S; ++s) {
+        float2 v[SP::R];
+        if (SP::read_slot(tid, s, a, c, buf, v)) SP::write_slot(tid, s, buf, v);
+    }
+}
+
+// The last pass: the buffer -> butterfly -> global memory.
+template <class K>
+SIP_HD void sk_ip_last(int tid, const TileArgs& a, const TileCtx& c, const float2* buf) {
+    if constexpr (K::OP == OP_R2C_HALF) {
+        sk_pair_last_r2c<K>(tid, a, c, buf);
+    } else if constexpr (K::OP == OP_R2C_PAIR) {
+        sk_pair_last_r2c_rows<K>(tid, a, c, buf);
+    } else {
+        using SP = SkPass<K, K::NP - 1>;
+#pragma unroll
+        for (int s = 0; s < SP::S; ++s) {
+            float2 v[SP::R];
+            if (SP::read_slot(tid, s, a, c, buf, v)) SP::store_slot(tid, s, a, c, v);
+        }
+    }
+}
+
+SIP_HD void sk_opaque(int& v) {
+#if defined(__CUDA_ARCH__)
+    asm volatile("" : "+r"(v));
+#else
+    (void)v;
+#endif
+}
+
+// A pulse tile's middle: the last forward pass leaves spectrum values
+// k + r N/R in a thread's registers, which is what the first inverse pass
+// (the transpose of the forward one: butterfly, then the conjugate twiddles)
+// takes, so the filter product happens there.
+template <class K>
+SIP_HD void sk_ip_turn(int tid, const TileArgs& a, const TileCtx& c, float2* buf) {
+    using SP = SkPass<K, K::NP - 1>;
+    constexpr int R = SP::R;
+    const bool cj = (a.flags & TF_MUL_CONJ) != 0;
+#pragma unroll 1
+    for (int s = 0; s < SP::S; ++s) {
+        const int b = tid + s * K::T;
+        if (SP::TOTAL % K::T != 0 && b >= SP::TOTAL) break;
+        int q, j;
+        SP::butterfly_index(b, q, j);
+        if (q >= c.cnt) continue;
+        float2* p = buf + SP::ip_slot(q, j);
+        float2 v[R], w[R], h[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = p[r * K::ip_step(K::NP - 1)];
+        sk_pass_twiddles<K, K::NP - 1>(a, c, j, w);
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = c_mul(v[r], w[r]);
+        // the filter comes from L2: its loads start before the butterfly
+        const float2* f = a.mul + (long long)(c.i0 + q) * a.mul_pitch_p + (long long)j * a.mul_pitch_k;
+        const long long step = SP::NR * a.mul_pitch_k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) h[r] = SIP_LDG(f + r * step);
+        dft<R, -1>(v);
+        if (cj) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) h[r].y = -h[r].y;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = c_mul(v[r], h[r]);
+        dft<R, 1>(v);
+        // read again (through an index the compiler does not know to be the
+        // same) rather than kept across both butterflies: 2 R registers
+        int j2 = j;
+        sk_opaque(j2);
+        sk_pass_twiddles<K, K::NP - 1>(a, c, j2, w);
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = c_mulc(v[r], w[r]);
+#pragma unroll
+        for (int r = 0; r < R; ++r) p[r * K::ip_step(K::NP - 1)] = v[r];
+    }
+}
+
+// Inverse pass of a pulse tile, in place (the transpose of forward pass
+// PASS); pass 0 has no twiddles and stores to global memory.
+template <class K, int PASS>
+SIP_HD void sk_ip_inverse(int tid, const TileArgs& a, const TileCtx& c, float2* buf) {
+    using SP = SkPass<K, PASS>;
+    constexpr int R = SP::R;
+#pragma unroll 1
+    for (int s = 0; s < SP::S; ++s) {
+        const int b = tid + s * K::T;
+        if (SP::TOTAL % K::T != 0 && b >= SP::TOTAL) break;
+        int q, j;
+        SP::butterfly_index(b, q, j);
+        if (q >= c.cnt) continue;
+        float2* p = buf + SP::ip_slot(q, j);
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = p[r * K::ip_step(PASS)];
+        dft<R, 1>(v);
+        if constexpr (PASS == 0) {
+            SkPass<SkView<K, OP_C2C, 1, true>, 0>::store_slot(tid, s, a, c, v);
+        } else {
+            int k, m;
+            SP::split_index(j, k, m);
+            float2 w[R];
+            sk_pass_twiddles<K, PASS>(a, c, k, w);
+#pragma unroll
+            for (int r = 1; r < R; ++r) v[r] = c_mulc(v[r], w[r]);
+#pragma unroll
+            for (int r = 0; r < R; ++r) p[r * K::ip_step(PASS)] = v[r];
+        }
+    }
+}
+
 }  // namespace sipfft
 
 // ------------------------------------------------------------ kernel
@@ -1568,6 +1920,24 @@ void sk_half(int tid, const TileArgs& a, const TileCtx& c, float2* buf) {
     sk_run<KV, 0>(tid, a, c, buf);
 }
 
+template <class K, int PASS>
+__device__ __forceinline__ void sk_ip_run_middle(int tid, const TileArgs& a, const TileCtx& c, float2* buf) {
+    if constexpr (PASS < K::NP - 1) {
+        sk_ip_middle<K, PASS>(tid, a, c, buf);
+        __syncthreads();
+        sk_ip_run_middle<K, PASS + 1>(tid, a, c, buf);
+    }
+}
+
+template <class K, int PASS>
+__device__ __forceinline__ void sk_ip_run_inverse(int tid, const TileArgs& a, const TileCtx& c, float2* buf) {
+    sk_ip_inverse<K, PASS>(tid, a, c, buf);
+    if constexpr (PASS > 0) {
+        __syncthreads();
+        sk_ip_run_inverse<K, PASS - 1>(tid, a, c, buf);
+    }
+}
+
 // STAGES = 2: the next tile is staged while the current one is transformed;
 // STAGES = 1: one buffer (tiles too large to double), overlap comes from
 // several CTAs per SM.
@@ -1579,6 +1949,54 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
     grid_dep_wait();
     grid_dep_launch();
     if (tile >= a.ntiles) return;
+    if constexpr (K::INPLACE) {
+        static_assert(STAGES == (K::SPLIT ? 2 : 1), "in-place tiles: the work buffer, behind the staged input if any");
+        using F = typename SkPick<K::OP == OP_PC, SkView<K, OP_PC, -1, false>, K>::type;
+        // work buffer first, then (after the twiddles) the staged input
+        float2* work = sk_smem;
+        float2* twp = sk_smem + K::BUF;
+        float2* stage = twp + K::TWSM;
+        sk_load_tws<K>(tid, a, twp);
+        if constexpr (K::SPLIT) {
+            sk_stage<K>(tid, a, decode_tile(a, tile), stage);
+            sk_commit();
+        } else if constexpr (K::TWS && K::TW2S > 0) {
+            __syncthreads();  // pass 0 reads staged real twiddles
+        }
+        for (; tile < a.ntiles; tile += gridDim.x) {
+            TileCtx c = decode_tile(a, tile);
+            c.tws = twp;
+            if constexpr (K::SPLIT) {
+                // one barrier: the input is there, the previous tile's last
+                // pass has read the work buffer
+                sk_wait<0>();
+                __syncthreads();
+                if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
+                    sk_zero_missing<K>(tid, a, c, stage);
+                    __syncthreads();
+                }
+                sk_ip_first<F>(tid, a, c, stage, work, [] {});
+                __syncthreads();
+                const int next = tile + gridDim.x;
+                if (next < a.ntiles) sk_stage<K>(tid, a, decode_tile(a, next), stage);
+                sk_commit();
+            } else {
+                // the barrier before the first write orders the staged
+                // twiddles and the previous tile's last reads
+                sk_ip_first<F>(tid, a, c, sk_ip_source<K>(a, c), work, [] { __syncthreads(); });
+                __syncthreads();
+            }
+            sk_ip_run_middle<F, 1>(tid, a, c, work);
+            if constexpr (K::OP == OP_PC) {
+                sk_ip_turn<K>(tid, a, c, work);
+                __syncthreads();
+                sk_ip_run_inverse<K, K::NP - 2>(tid, a, c, work);
+            } else {
+                sk_ip_last<K>(tid, a, c, work);
+            }
+        }
+        return;
+    }
     // staged twiddles after the buffers (the barrier before pass 0 of the
     // first tile orders the copy before any use)
     float2* tws = sk_smem + (STAGES == 2 ? 2 : 1) * K::BUF;
@@ -1590,7 +2008,7 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
         sk_commit();
         for (; tile < a.ntiles; tile += gridDim.x) {
             TileCtx c = decode_tile(a, tile);
-            if constexpr (K::TWS) c.tws = tws;
+            c.tws = tws;
             sk_wait<0>();
             __syncthreads();
             if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
@@ -1615,7 +2033,7 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
     for (int it = 0; tile < a.ntiles; ++it, tile += gridDim.x) {
         float2* cur = bufs[it & 1];
         TileCtx c = decode_tile(a, tile);
-        if constexpr (K::TWS) c.tws = tws;
+        c.tws = tws;
         if (STAGES == 2) {
             const int next = tile + gridDim.x;
             if (next < a.ntiles) sk_stage<K>(tid, a, decode_tile(a, next), bufs[(it + 1) & 1]);

@@ -27,7 +27,10 @@ enum SkMode : int {
 //                   layout into the other buffer, one butterfly (pair) at a
 //                   time instead of all of them across a barrier; the next
 //                   tile is staged after pass 0 (overlapping the later
-//                   passes) instead of before it.
-enum : int { SK_TW_BASIS = 1, SK_TW_SMEM = 2, SK_MIRROR_PAIR = 4, SK_SPLIT_PASS0 = 8 };
+//                   passes) instead of before it;
+//   SK_IN_PLACE     no staging: pass 0 reads global memory, and every later
+//                   pass reads and writes the same slots of the tile's one
+//                   buffer (sk_kernel.cuh, "in-place passes").
+enum : int { SK_TW_BASIS = 1, SK_TW_SMEM = 2, SK_MIRROR_PAIR = 4, SK_SPLIT_PASS0 = 8, SK_IN_PLACE = 16 };
 
 }  // namespace sipfft

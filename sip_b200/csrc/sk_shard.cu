@@ -28,7 +28,7 @@ SkEntry make_entry(std::vector<int> radices) {
     e.stages = STAGES;
     e.radices = std::move(radices);
     e.LD = K::LD;
-    e.smem = (STAGES == 2 ? 2 : 1) * K::BUF * 8 + K::TWSM * 8;
+    e.smem = K::smem_bytes(STAGES);
     e.fn = reinterpret_cast<const void*>(&sk_fft_kernel<K, STAGES>);
     e.minb = K::MINB;
     return e;

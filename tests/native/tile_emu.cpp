@@ -152,8 +152,55 @@ void emu_sk_passes(const TileArgs& a, const TileCtx& c, float2* buf) {
     }
 }
 
+// ---- in-place tiles (SK_IN_PLACE): the same phase functions per thread
+template <class K, int PASS>
+void emu_ip_middle(const TileArgs& a, const TileCtx& c, float2* buf) {
+    if constexpr (PASS < K::NP - 1) {
+        for (int tid = 0; tid < K::T; ++tid) sk_ip_middle<K, PASS>(tid, a, c, buf);
+        emu_ip_middle<K, PASS + 1>(a, c, buf);
+    }
+}
+
+template <class K, int PASS>
+void emu_ip_inverse(const TileArgs& a, const TileCtx& c, float2* buf) {
+    for (int tid = 0; tid < K::T; ++tid) sk_ip_inverse<K, PASS>(tid, a, c, buf);
+    if constexpr (PASS > 0) emu_ip_inverse<K, PASS - 1>(a, c, buf);
+}
+
+template <class K>
+void emu_ip_run(const TileArgs& a) {
+    const float nan = std::numeric_limits<float>::quiet_NaN();
+    std::vector<float2> buf(K::BUF), tws(K::TWSM + 1, make_float2(nan, nan));
+    for (int tid = 0; tid < K::T; ++tid) sk_load_tws<K>(tid, a, tws.data());
+    using F = typename SkPick<K::OP == OP_PC, SkView<K, OP_PC, -1, false>, K>::type;
+    for (int tile = 0; tile < a.ntiles; ++tile) {
+        TileCtx c = decode_tile(a, tile);
+        c.tws = tws.data();
+        for (auto& v : buf) v = make_float2(nan, nan);
+        if constexpr (K::SPLIT) {
+            std::vector<float2> stage(K::STAGE + 2, make_float2(nan, nan));
+            for (int tid = 0; tid < K::T; ++tid) sk_stage<K>(tid, a, c, stage.data());
+            for (int tid = 0; tid < K::T; ++tid) sk_zero_missing<K>(tid, a, c, stage.data());
+            for (int tid = 0; tid < K::T; ++tid) sk_ip_first<F>(tid, a, c, stage.data(), buf.data(), [] {});
+        } else {
+            for (int tid = 0; tid < K::T; ++tid)
+                sk_ip_first<F>(tid, a, c, sk_ip_source<K>(a, c), buf.data(), [] {});
+        }
+        emu_ip_middle<F, 1>(a, c, buf.data());
+        if constexpr (K::OP == OP_PC) {
+            for (int tid = 0; tid < K::T; ++tid) sk_ip_turn<K>(tid, a, c, buf.data());
+            emu_ip_inverse<K, K::NP - 2>(a, c, buf.data());
+        } else {
+            for (int tid = 0; tid < K::T; ++tid) sk_ip_last<K>(tid, a, c, buf.data());
+        }
+    }
+}
+
 template <class K>
 void emu_sk_run(const TileArgs& a) {
+    if constexpr (K::INPLACE) {
+        emu_ip_run<K>(a);
+    } else {
     const float nan = std::numeric_limits<float>::quiet_NaN();
     std::vector<float2> buf(K::BUF);
     // staged twiddles (SK_TW_SMEM), NaN where the copy does not write
@@ -161,7 +208,7 @@ void emu_sk_run(const TileArgs& a) {
     for (int tid = 0; tid < K::T; ++tid) sk_load_tws<K>(tid, a, tws.data());
     for (int tile = 0; tile < a.ntiles; ++tile) {
         TileCtx c = decode_tile(a, tile);
-        if constexpr (K::TWS) c.tws = tws.data();
+        c.tws = tws.data();
         for (auto& v : buf) v = make_float2(nan, nan);
         for (int tid = 0; tid < K::T; ++tid) sk_stage<K>(tid, a, c, buf.data());
         for (int tid = 0; tid < K::T; ++tid) sk_zero_missing<K>(tid, a, c, buf.data());
@@ -182,6 +229,7 @@ void emu_sk_run(const TileArgs& a) {
         emu_sk_passes<K, 0>(a, c, buf.data());
         if constexpr (sk_last_to_smem<K>())
             for (int tid = 0; tid < K::T; ++tid) sk_post<K>(tid, a, c, buf.data());
+    }
     }
 }
 
@@ -273,7 +321,7 @@ SkEntry emu_entry(std::vector<int> radices) {
     e.stages = STAGES;
     e.radices = std::move(radices);
     e.LD = K::LD;
-    e.smem = (STAGES == 2 ? 2 : 1) * K::BUF * 8 + K::TWSM * 8;
+    e.smem = K::smem_bytes(STAGES);
     e.fn = reinterpret_cast<const void*>(&emu_sk_run<K>);
     return e;
 }
@@ -288,9 +336,14 @@ const std::vector<SkEntry>& sk_registry() {
     v.push_back(emu_entry<SkCfg<N, P, T, OP, MODE, SIGN, TW4, MINB, TWB, __VA_ARGS__>, STAGES>({__VA_ARGS__}));
         SIP_SK_CONFIGS(SIP_EMU_SK)
         // Pulse-compression tiles (the library compiles these at run time,
-        // csrc/jit.cpp): rows of 1000, Bluestein's 2025 for n = 1009, and the
-        // four-step pass P (cross twiddles) of 2^18 = 512 x 512 and of
+        // csrc/jit.cpp, in place): rows of 1000, Bluestein's 2025 for n = 1009,
+        // and the four-step pass P (cross twiddles) of 2^18 = 512 x 512 and of
         // Bluestein's 40500 = 180 x 225 for n = 20011.
+        SIP_EMU_SK(0, 1000, 4, 128, OP_PC, SK_ROWS, 1, false, 1, 4, 17, 10, 10, 10)
+        SIP_EMU_SK(0, 2025, 2, 128, OP_PC, SK_ROWS, 1, false, 1, 4, 19, 15, 15, 9)
+        SIP_EMU_SK(0, 512, 8, 128, OP_PC, SK_ROWS, 1, true, 1, 4, 17, 32, 16)
+        SIP_EMU_SK(0, 225, 16, 128, OP_PC, SK_ROWS, 1, true, 1, 4, 17, 15, 15)
+        // The self-sorting form (the library's for one-pass lengths) as variant 1.
         SIP_EMU_SK(0, 1000, 4, 128, OP_PC, SK_ROWS, 1, false, 2, 4, 1, 10, 10, 10)
         SIP_EMU_SK(0, 2025, 2, 192, OP_PC, SK_ROWS, 1, false, 2, 2, 1, 15, 15, 9)
         SIP_EMU_SK(0, 512, 8, 256, OP_PC, SK_ROWS, 1, true, 2, 2, 1, 32, 16)
