@@ -117,7 +117,7 @@ BufPtr root_table(int device, long long n, long long count) {
 
 BufPtr split_table(int device, long long n, int shift) {
     const long long B = 1LL << shift;
-    const long long count = B + (n + B - 1) / B;
+    const long long count = 6 * B;  // 2 B single and 2 B double precision values (B >= sqrt(n))
     TableKey key{device, 3, n, shift, {}};
     std::lock_guard<std::mutex> lk(g_table_mu);
     auto it = g_tables.find(key);

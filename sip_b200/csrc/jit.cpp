@@ -366,10 +366,11 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     const long long buf =
         8LL * (inplace ? sk_ip_buffer_values(c.P, lay) : sk_buffer_values(op, c.P, n, r0, c.twb));
     const long long staged = 8LL * ((sk_stage_slots(op, c.P, n, c.twb) + 1) / 2 * 2);  // in-place tiles' input
-    long long tws = 8LL * sk_tws_values(op, n, c.radices.data(), (int)c.radices.size(), c.twb);
+    const long long cross = 8LL * sk_cross_values(op, tw4, c.P, c.radices.data(), (int)c.radices.size(), c.twb);
+    long long tws = cross + 8LL * sk_tws_values(op, n, c.radices.data(), (int)c.radices.size(), c.twb);
     if (buf + tws > kMaxTileSmem && (c.twb & SK_TW_SMEM)) {  // no room for the staged twiddles
         c.twb &= ~SK_TW_SMEM;
-        tws = 0;
+        tws = cross;
     }
     const long long both = inplace ? buf + ((c.twb & SK_SPLIT_PASS0) ? staged : 0) : 2 * buf;
     if (inplace && (!(c.twb & SK_SPLIT_PASS0) || both + tws > kMaxTileSmem)) c.stages = 1;

@@ -142,6 +142,12 @@ SIP_HD constexpr int sk_tws_values(int op, int n, const int* rs, int np, int fla
     return (flags & SK_TW_SMEM) ? (total + 1) / 2 * 2 : 0;
 }
 
+// Complex values of the cross twiddle table of a four-step tile (even count).
+SIP_HD constexpr int sk_cross_values(int op, bool tw4, int p, const int* rs, int np, int flags) {
+    const int r = (flags & SK_IN_PLACE) && op == OP_PC ? rs[0] : rs[np - 1];
+    return tw4 ? (p * r + 1) / 2 * 2 : 0;
+}
+
 // Staged input values (complex64 units) per tile.
 SIP_HD constexpr int sk_stage_values(int op, int p, int n) {
     return op == OP_C2R_HALF ? p * (n + 1)
@@ -259,10 +265,15 @@ struct SkCfg {
     static constexpr int TW2_OFF = tws_off(NP);
     static constexpr int TW2S = sk_tw2s(CFG_OP, N, radix(0), radix(NP - 1), FLAGS);
     static constexpr int TWSM = TWS ? (TW2_OFF + TW2S + 1) / 2 * 2 : 0;
+    // Cross twiddle table of a four-step tile (sk_load_cross), behind them;
+    // XR is the radix of the pass that stores (pass 0 for an in-place pulse tile).
+    static constexpr int XR = INPLACE && OP == OP_PC ? radix(0) : radix(NP - 1);
+    static constexpr int XTW = sk_cross_values(OP, TW4, P, rad_list, NP, FLAGS);
+    static constexpr int TWS_ALL = TWSM + XTW;
     // Dynamic shared memory (bytes) of the kernel with STAGES buffers.
     static constexpr int smem_bytes(int stages) {
         return 8 * ((INPLACE ? BUF + (SPLIT ? (sk_stage_slots(OP, P, N, FLAGS) + 1) / 2 * 2 : 0) : stages * BUF) +
-                    TWSM);
+                    TWS_ALL);
     }
     // CTAs per SM the shared memory allows with two stages (228 KB per SM,
     // 1 KB reserved per CTA); used as the register-allocation target.
@@ -745,6 +756,45 @@ SIP_HD void sk_static_for(F&& f) {
     }
 }
 
+// ---------------------------------------------------- cross twiddles
+// W_N^m from the double-precision copy of the split table (behind the single
+// one, twiddle.cu k_split_tw), rounded once.
+SIP_HD float2 sk_cross_tw(const TileArgs& a, long long m) {
+    const long long B = 1LL << a.tw4_shift;
+    const double2* t = reinterpret_cast<const double2*>(a.tw2 + 2 * B);
+    const double2 lo = SIP_LDG(t + (m & (B - 1))), hi = SIP_LDG(t + B + (m >> a.tw4_shift));
+    return make_float2((float)(lo.x * hi.x - lo.y * hi.y), (float)(lo.x * hi.y + lo.y * hi.x));
+}
+
+// Four-step cross twiddle of element k = j + r NR of transform c = i0 + q:
+// W_N^{c k} = W_N^{c j} (W_N^{c NR})^r.  The first factor is one per butterfly;
+// the second depends on (q, r) alone and comes from a table of P x R values
+// made once per tile behind the staged twiddles.  Both are rounded once, so
+// their product is as accurate as the product of two split-table entries
+// that every element looked up before: two 64-bit index computations and
+// loads per value, which made the column pass of C2C 65536 x 4096 30 % slower
+// than its row pass.
+template <class K>
+SIP_HD void sk_load_cross(int tid, const TileArgs& a, const TileCtx& c, float2* xtw) {
+    if constexpr (K::TW4) {
+        constexpr int R = K::XR, NR = K::N / R;
+        for (int i = tid; i < K::P * R; i += K::T) {
+            const int r = i / K::P, q = i - r * K::P;
+            if (q < c.cnt) xtw[i] = sk_cross_tw(a, (long long)(c.i0 + q) * (r * NR));
+        }
+    }
+}
+
+template <class K, int R, int NR>
+SIP_HD void sk_cross(const TileArgs& a, const TileCtx& c, int q, int j, float2 (&v)[R]) {
+    static_assert(R == K::XR, "the table is made for the storing pass");
+    const float2 w0 = sk_cross_tw(a, (long long)(c.i0 + q) * j);
+    const float2* t = c.tws + K::TWSM + q;
+    v[0] = c_tw<K::SIGN>(v[0], w0);
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = c_tw<K::SIGN>(v[r], c_mul(w0, t[r * K::P]));
+}
+
 // ------------------------------------------------------------- passes
 template <class K, int PASS>
 struct SkPass {
@@ -889,11 +939,7 @@ struct SkPass {
         if (!K::MIRROR && q >= c.cnt) return;
         if constexpr (K::OP == OP_C2C) {
             const bool blue = K::WORK_IN && (a.flags & TF_BLUE) != 0;
-            if constexpr (K::TW4) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    v[r] = c_tw<K::SIGN>(v[r], cross_tw(a, (long long)(c.i0 + q) * (j + r * NR)));
-            }
+            if constexpr (K::TW4) sk_cross<K, R, NR>(a, c, q, j, v);
             if (blue) {  // Bluestein: outputs k < n_other times the chirp
 #pragma unroll
                 for (int r = 0; r < R; ++r)
@@ -1955,7 +2001,7 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
         // work buffer first, then (after the twiddles) the staged input
         float2* work = sk_smem;
         float2* twp = sk_smem + K::BUF;
-        float2* stage = twp + K::TWSM;
+        float2* stage = twp + K::TWS_ALL;
         sk_load_tws<K>(tid, a, twp);
         if constexpr (K::SPLIT) {
             sk_stage<K>(tid, a, decode_tile(a, tile), stage);
@@ -1975,6 +2021,7 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
                     sk_zero_missing<K>(tid, a, c, stage);
                     __syncthreads();
                 }
+                sk_load_cross<K>(tid, a, c, twp + K::TWSM);
                 sk_ip_first<F>(tid, a, c, stage, work, [] {});
                 __syncthreads();
                 const int next = tile + gridDim.x;
@@ -1984,6 +2031,7 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
                 // the barrier before the first write orders the staged
                 // twiddles and the previous tile's last reads
                 sk_ip_first<F>(tid, a, c, sk_ip_source<K>(a, c), work, [] { __syncthreads(); });
+                sk_load_cross<K>(tid, a, c, twp + K::TWSM);
                 __syncthreads();
             }
             sk_ip_run_middle<F, 1>(tid, a, c, work);
@@ -2011,6 +2059,7 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
             c.tws = tws;
             sk_wait<0>();
             __syncthreads();
+            sk_load_cross<K>(tid, a, c, tws + K::TWSM);
             if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
                 sk_zero_missing<K>(tid, a, c, bufs[0]);
                 __syncthreads();
@@ -2045,6 +2094,7 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
             sk_wait<0>();
         }
         __syncthreads();
+        sk_load_cross<K>(tid, a, c, tws + K::TWSM);
         if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
             sk_zero_missing<K>(tid, a, c, cur);
             __syncthreads();

@@ -69,20 +69,26 @@ __global__ void k_root_tw(float2* out, long long n, long long count) {
         out[i] = root_fwd(i, n);
 }
 
-// Split cross-twiddle table: [W_n^lo, lo < B][W_n^{hi B}, hi < ceil(n/B)].
-__global__ void k_split_tw(float2* out, long long n, long long B, long long count) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
-         i += (long long)gridDim.x * blockDim.x)
-        out[i] = root_fwd(i < B ? i : (i - B) * B, n);
+// Split cross-twiddle table: [W_n^lo, lo < B][W_n^{hi B}, hi < B], then the same
+// 2 B values in double precision (sk_kernel.cuh sk_cross_tw).
+__global__ void k_split_tw(float2* out, long long n, long long B) {
+    double2* d = reinterpret_cast<double2*>(out + 2 * B);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < 2 * B;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long m = i < B ? i : (i - B) * B;
+        out[i] = root_fwd(m, n);
+        double s, c;
+        sincospi(2.0 * (double)(m % n) / (double)n, &s, &c);
+        d[i] = make_double2(c, -s);
+    }
 }
 
 }  // namespace
 
 cudaError_t gen_split_twiddles(float2* out, long long n, int shift, cudaStream_t stream) {
     const long long B = 1LL << shift;
-    const long long count = B + (n + B - 1) / B;
     const int block = 256;
-    k_split_tw<<<(unsigned)((count + block - 1) / block), block, 0, stream>>>(out, n, B, count);
+    k_split_tw<<<(unsigned)((2 * B + block - 1) / block), block, 0, stream>>>(out, n, B);
     return cudaGetLastError();
 }
 

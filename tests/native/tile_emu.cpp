@@ -71,7 +71,14 @@ std::vector<float2> tw2_host(const Step& st) {
         for (long long k = 0; k < st.tw2_count; ++k) t.push_back(root_host(k, st.tw2_n));
     } else if (st.tw2_kind == 2) {
         const long long B = 1LL << st.L.args.tw4_shift;
-        for (long long k = 0; k < st.tw2_count; ++k) t.push_back(root_host(k < B ? k : (k - B) * B, st.tw2_n));
+        t.assign(6 * B, make_float2(0.f, 0.f));
+        double2* d = reinterpret_cast<double2*>(t.data() + 2 * B);
+        for (long long k = 0; k < 2 * B; ++k) {
+            const long long m = (k < B ? k : (k - B) * B) % st.tw2_n;
+            t[k] = root_host(m, st.tw2_n);
+            const long double x = 2.0L * 3.141592653589793238462643383279502884L * (long double)m / (long double)st.tw2_n;
+            d[k] = make_double2((double)std::cos(x), (double)(-std::sin(x)));
+        }
     }
     return t;
 }
@@ -170,13 +177,14 @@ void emu_ip_inverse(const TileArgs& a, const TileCtx& c, float2* buf) {
 template <class K>
 void emu_ip_run(const TileArgs& a) {
     const float nan = std::numeric_limits<float>::quiet_NaN();
-    std::vector<float2> buf(K::BUF), tws(K::TWSM + 1, make_float2(nan, nan));
+    std::vector<float2> buf(K::BUF), tws(K::TWS_ALL + 1, make_float2(nan, nan));
     for (int tid = 0; tid < K::T; ++tid) sk_load_tws<K>(tid, a, tws.data());
     using F = typename SkPick<K::OP == OP_PC, SkView<K, OP_PC, -1, false>, K>::type;
     for (int tile = 0; tile < a.ntiles; ++tile) {
         TileCtx c = decode_tile(a, tile);
         c.tws = tws.data();
         for (auto& v : buf) v = make_float2(nan, nan);
+        for (int tid = 0; tid < K::T; ++tid) sk_load_cross<K>(tid, a, c, tws.data() + K::TWSM);
         if constexpr (K::SPLIT) {
             std::vector<float2> stage(K::STAGE + 2, make_float2(nan, nan));
             for (int tid = 0; tid < K::T; ++tid) sk_stage<K>(tid, a, c, stage.data());
@@ -204,12 +212,13 @@ void emu_sk_run(const TileArgs& a) {
     const float nan = std::numeric_limits<float>::quiet_NaN();
     std::vector<float2> buf(K::BUF);
     // staged twiddles (SK_TW_SMEM), NaN where the copy does not write
-    std::vector<float2> tws(K::TWSM + 1, make_float2(nan, nan));
+    std::vector<float2> tws(K::TWS_ALL + 1, make_float2(nan, nan));
     for (int tid = 0; tid < K::T; ++tid) sk_load_tws<K>(tid, a, tws.data());
     for (int tile = 0; tile < a.ntiles; ++tile) {
         TileCtx c = decode_tile(a, tile);
         c.tws = tws.data();
         for (auto& v : buf) v = make_float2(nan, nan);
+        for (int tid = 0; tid < K::T; ++tid) sk_load_cross<K>(tid, a, c, tws.data() + K::TWSM);
         for (int tid = 0; tid < K::T; ++tid) sk_stage<K>(tid, a, c, buf.data());
         for (int tid = 0; tid < K::T; ++tid) sk_zero_missing<K>(tid, a, c, buf.data());
         if constexpr (K::SPLIT) {  // pass 0 from the staging buffer into a separate work buffer
