@@ -155,6 +155,18 @@ std::vector<int> jit_pulse_radices(int n) {
     return best.empty() ? jit_radices(n) : best;
 }
 
+// The factorization an operation's tiles use, found once per length (plans
+// are made per request by some programs).
+const std::vector<int>& tile_radices(int op, int n) {
+    static std::mutex& mu = *new std::mutex;
+    static auto& known = *new std::map<std::pair<bool, int>, std::vector<int>>;
+    const auto key = std::make_pair(op == OP_PC, n);
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = known.find(key);
+    if (it == known.end()) it = known.emplace(key, op == OP_PC ? jit_pulse_radices(n) : jit_radices(n)).first;
+    return it->second;
+}
+
 // sk_ip_layout, searched once per radix order, tile and mode.
 SkIpLayout ip_layout(const std::vector<int>& radices, int P, int mode) {
     static std::mutex& mu = *new std::mutex;
@@ -296,7 +308,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     c.sign = sign;
     c.tw4 = tw4;
     c.n = n;
-    c.radices = order != nullptr ? *order : op == OP_PC ? jit_pulse_radices(n) : jit_radices(n);
+    c.radices = order != nullptr ? *order : tile_radices(op, n);
     // Tuning overrides (sweeps; unset in normal use): SIP_FFT_JIT_RADICES
     // ("25,15,8", must multiply to n), SIP_FFT_JIT_P, SIP_FFT_JIT_T,
     // SIP_FFT_JIT_MINB, SIP_FFT_JIT_STAGES, SIP_FFT_JIT_TWB (the SK_TW_* bits
@@ -321,12 +333,77 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     }
     if (c.radices.empty()) return false;
     transforms = std::max<long long>(1, transforms);
-    // transforms per tile: about SIP_FFT_JIT_TILE (4096) values for rows,
-    // runs of 16 adjacent transforms (128-byte segments) for the column
-    // modes; at most SIP_FFT_JIT_E (32) values per thread and pass
+    // Twiddle and pass options (SK_* bits; SIP_FFT_JIT_TWB overrides them): the
+    // basis table staged in shared memory and a split pass 0 (dropped below
+    // where they do not apply), and
+    //  - from three passes on, in place: one barrier per pass and one
+    //    butterfly live per thread, so that no tile spills.  C2C rows of 33.5 M
+    //    values: 1200 as 12 x 10 x 10 103 us against 138, 3000 111 against
+    //    150, 5000 134 against 162, 9000 156 against 182.  Two passes have one
+    //    exchange, and the self-sorting form is as fast or faster (420 as
+    //    21 x 20: 94 us against 107).
+    //  - R2C: in place too, on mirrored butterfly pairs, also for two passes
+    //    whose pairs fit the registers (last radix up to 21): rows of 504
+    //    111 us against 144, 2400 126 against 183, 10000 134 against 191; 1250
+    //    as 25 x 25 150 self-sorting against 186.
+    //  - C2R row pairs only above 5000 values (one tile of two rows is then
+    //    most of an SM's shared memory): 6561 171 against 183, 12005 219
+    //    against 288; 945 135 against 128, 3375 150 against 141.
+    const size_t passes = c.radices.size();
+    int options = SK_TW_BASIS | SK_TW_SMEM | SK_SPLIT_PASS0;
+    if (op == OP_PC) options = SK_TW_BASIS | SK_IN_PLACE;
+    else if (op == OP_R2C_HALF || op == OP_R2C_PAIR) {
+        if (passes >= 3 || c.radices.back() <= 21) options |= SK_IN_PLACE | SK_MIRROR_PAIR;
+    } else if (passes >= 3 && (op != OP_C2R_PAIR || n > 5000)) options |= SK_IN_PLACE;
+    options = ovr_int("SIP_FFT_JIT_TWB", options);
+    if (options < 0 || options > 31) return false;
+    if ((options & SK_MIRROR_PAIR) && (!real_op || passes < 2)) options &= ~SK_MIRROR_PAIR;
+    if (passes < 2) options &= ~(SK_IN_PLACE | SK_SPLIT_PASS0);
+    const bool inplace = (options & SK_IN_PLACE) != 0;
+    if (op == OP_PC && !inplace) options &= ~SK_SPLIT_PASS0;
+    if (inplace && (op == OP_R2C_HALF || op == OP_R2C_PAIR)) options |= SK_MIRROR_PAIR;
+
+    // Shared memory of a tile of P transforms: work buffer, the input staged
+    // beside it, cross and staged twiddles.
+    struct Bytes {
+        long long buf, staged, cross, tws;
+    };
+    auto bytes = [&](int P, SkIpLayout* lay) {
+        const int* rs = c.radices.data();
+        Bytes s{};
+        if (inplace) {
+            *lay = ip_layout(c.radices, P, mode);
+            s.buf = 8LL * sk_ip_buffer_values(P, *lay);
+            s.staged = (options & SK_SPLIT_PASS0) ? 8LL * ((sk_stage_slots(op, P, n, options) + 1) / 2 * 2) : 0;
+        } else {
+            s.buf = 8LL * sk_buffer_values(op, P, n, rs[0], options);
+            s.staged = s.buf;  // the second buffer
+        }
+        s.cross = 8LL * sk_cross_values(op, tw4, P, rs, (int)passes, options);
+        s.tws = 8LL * sk_tws_values(op, n, rs, (int)passes, options);
+        return s;
+    };
+    SkIpLayout lay{0, 0, 0};
+
+    // transforms per tile: about SIP_FFT_JIT_TILE (4096) values for rows, runs
+    // of 16 adjacent transforms (128-byte segments) for the column modes, 8 or
+    // 4 where only those leave room for staging the next tile's input (33.5 M
+    // values in columns of 1000: 140 us with 8, 203 with 16 and no room;
+    // 2048: 176 us with 4, 193 with 8); at most SIP_FFT_JIT_E (32) values
+    // per thread and pass
     const int tile_values = std::max(64, env_int("SIP_FFT_JIT_TILE", 4096));
     const int per_thread = std::max(8, values > 0 ? values : env_int("SIP_FFT_JIT_E", 32));
-    long long P = mode == SK_ROWS ? std::max(1, tile_values / n) : 16;
+    long long P = std::max(1, tile_values / n);
+    if (mode != SK_ROWS) {
+        P = 16;
+        for (int p = 16; p >= 4; p /= 2) {
+            const Bytes s = bytes(p, &lay);
+            if (s.buf + s.staged + s.cross <= kMaxTileSmem) {
+                P = p;
+                break;
+            }
+        }
+    }
     P = std::min<long long>(P, transforms);
     int T = 0;
     for (;;) {
@@ -340,47 +417,29 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     if (ovr_int("SIP_FFT_JIT_T", 0) > 0) T = ovr_int("SIP_FFT_JIT_T", 0);
     if (T % 32 != 0 || T > kMaxTileThreads) return false;
     c.P = (int)P;
-    c.T = T;
-    const int r0 = c.radices[0];
-    c.LD = sk_pitch(n, r0);
-    // twiddle options (SK_TW_* bits; SIP_FFT_JIT_TWB overrides them).  By
-    // default the basis table staged in shared memory and a split pass 0
-    // (dropped below where they do not apply): 3-23 % faster on B200 than
-    // the basis table through L1 over run-time compiled C2C rows of 544 to
-    // 8160 points.  Mirrored butterfly pairs (on request) apply to real
-    // half-length tiles of two or more passes.
-    c.twb = ovr_int("SIP_FFT_JIT_TWB", op == OP_PC ? SK_TW_BASIS | SK_IN_PLACE
-                                                   : SK_TW_BASIS | SK_TW_SMEM | SK_SPLIT_PASS0);
-    if (c.twb < 0 || c.twb > 31) return false;
-    if ((c.twb & SK_MIRROR_PAIR) && (!real_op || c.radices.size() < 2)) c.twb &= ~SK_MIRROR_PAIR;
-    if ((c.twb & SK_SPLIT_PASS0) && (c.radices.size() < 2 || (op == OP_PC && !(c.twb & SK_IN_PLACE))))
-        c.twb &= ~SK_SPLIT_PASS0;
-    if (c.radices.size() < 2) c.twb &= ~SK_IN_PLACE;
-    const bool inplace = (c.twb & SK_IN_PLACE) != 0;
-    if (inplace && (op == OP_R2C_HALF || op == OP_R2C_PAIR)) c.twb |= SK_MIRROR_PAIR;
-    SkIpLayout lay{0, 0};
-    if (inplace) {
-        lay = ip_layout(c.radices, c.P, mode);
-        c.LD = lay.ld;
+    c.twb = options;
+    const Bytes s = bytes(c.P, &lay);
+    c.LD = inplace ? lay.ld : sk_pitch(n, c.radices[0]);
+    auto ctas = [](long long b) { return (int)std::max(1LL, (228 * 1024) / (b + 1024)); };
+    // The staged twiddles give way to the staged input, and to a second CTA
+    // per SM (C2C rows of 7000: 146 us with two CTAs of 256 threads and the
+    // twiddles through L1, 154 with one of 352).
+    const long long input = s.buf + s.staged + s.cross;
+    bool second_cta = false;
+    if (c.twb & SK_TW_SMEM) {
+        const bool fits = inplace ? input > kMaxTileSmem || input + s.tws <= kMaxTileSmem
+                                  : s.buf + s.cross + s.tws <= kMaxTileSmem;
+        second_cta = inplace && s.staged > 0 && ctas(input) == 2 && ctas(input + s.tws) == 1;
+        if (!fits || s.buf + s.cross + s.tws > kMaxTileSmem || second_cta) c.twb &= ~SK_TW_SMEM;
     }
-    const long long buf =
-        8LL * (inplace ? sk_ip_buffer_values(c.P, lay) : sk_buffer_values(op, c.P, n, r0, c.twb));
-    const long long staged = 8LL * ((sk_stage_slots(op, c.P, n, c.twb) + 1) / 2 * 2);  // in-place tiles' input
-    const long long cross = 8LL * sk_cross_values(op, tw4, c.P, c.radices.data(), (int)c.radices.size(), c.twb);
-    long long tws = cross + 8LL * sk_tws_values(op, n, c.radices.data(), (int)c.radices.size(), c.twb);
-    if (buf + tws > kMaxTileSmem && (c.twb & SK_TW_SMEM)) {  // no room for the staged twiddles
-        c.twb &= ~SK_TW_SMEM;
-        tws = cross;
-    }
-    const long long both = inplace ? buf + ((c.twb & SK_SPLIT_PASS0) ? staged : 0) : 2 * buf;
-    if (inplace && (!(c.twb & SK_SPLIT_PASS0) || both + tws > kMaxTileSmem)) c.stages = 1;
-    else if (both + tws <= kMaxTileSmem) c.stages = 2;
-    else if (buf + tws <= kMaxTileSmem) c.stages = 1;
-    else return false;
+    const long long tws = s.cross + ((c.twb & SK_TW_SMEM) ? s.tws : 0);
+    if (s.buf + tws > kMaxTileSmem) return false;
+    c.stages = s.staged > 0 && s.buf + s.staged + tws <= kMaxTileSmem ? 2 : 1;
     if (ovr_int("SIP_FFT_JIT_STAGES", 0) == 1) c.stages = 1;
-    if (c.stages != 2) c.twb &= ~SK_SPLIT_PASS0;  // a split pass 0 uses the second buffer as its work layout
-    if (inplace && buf + tws > kMaxTileSmem) return false;
-    c.smem = (int)((c.stages == 2 ? both : buf) + tws);
+    if (c.stages != 2) c.twb &= ~SK_SPLIT_PASS0;  // a split pass 0 needs the staged input beside the work buffer
+    c.smem = (int)(s.buf + (c.stages == 2 ? s.staged : 0) + tws);
+    if (second_cta && c.stages == 2 && ovr_int("SIP_FFT_JIT_T", 0) == 0) T = std::min(T, 256);
+    c.T = T;
     const int smem_ctas = std::max<int>(1, (228 * 1024) / (c.smem + 1024));
     c.minb = std::max(1, std::min(65536 / (T * 128), smem_ctas));
     if (inplace && op == OP_PC) {
@@ -392,7 +451,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
         // threads, 251 with 2 of 256, 328 with 1 of 288; 8640: 248 us with 2 of
         // 256, 326 with 1 of 384.  `values` other than 32: half the CTAs, for
         // tiles that spill.
-        const int fit = std::max<int>(1, (228 * 1024) / ((int)(buf + tws) + 1024));
+        const int fit = ctas(s.buf + tws);
         c.T = fit >= 4 ? 128 : fit >= 2 ? 256 : 512;
         c.minb = std::max(1, std::min(fit, 512 / c.T) / (per_thread == 32 ? 1 : 2));
         if (ovr_int("SIP_FFT_JIT_T", 0) > 0) c.T = ovr_int("SIP_FFT_JIT_T", 0);
@@ -563,7 +622,7 @@ std::vector<JitCfg> jit_candidates(int op, int mode, int sign, bool tw4, int n, 
     // fits in the registers without spills varies (a pulse tile of 4320
     // points as 18 x 16 x 15 on 288 threads spills 240 bytes per thread,
     // as 15 x 16 x 18 none)
-    std::vector<std::vector<int>> orders = {op == OP_PC ? jit_pulse_radices(n) : jit_radices(n)};
+    std::vector<std::vector<int>> orders = {tile_radices(op, n)};
     if (!orders[0].empty() && orders[0].front() != orders[0].back())
         orders.push_back(std::vector<int>(orders[0].rbegin(), orders[0].rend()));
     for (size_t oi = 0; oi < orders.size(); ++oi)

@@ -4,7 +4,8 @@
 // that the kernel does not spill.  TWB holds the sk_kernel.cuh SK_* bits:
 // 1 basis (else full) pass twiddles, 2 twiddles staged in shared memory,
 // 4 mirrored butterfly pairs in the real tiles' last (R2C) or first (C2R)
-// pass, 8 pass 0 from the staging buffer into a separate work buffer.
+// pass, 8 pass 0 from the staging buffer into a separate work buffer, 16 passes
+// in place (one barrier per pass, one butterfly live per thread).
 // Every other length runs on the generic tile kernel.  The shard index
 // spreads the instantiations over parallel compile units.  Several entries
 // for the same (N, OP, MODE, SIGN, TW4) are variants of the tile shape or
@@ -13,26 +14,30 @@
 #pragma once
 
 #define SIP_SK_CONFIGS(X)                                                     \
-    /* 1D / last-axis C2C rows (split pass 0, TWB 9) */                       \
+    /* 1D / last-axis C2C rows (split pass 0, TWB 9; in place with staged     \
+       input: 1024 as 32 x 32 87.5 us per 33.5 M values against 103           \
+       self-sorting as 16 x 16 x 4, 8192 with staged twiddles 115 against     \
+       140) */                                                                \
     X(0, 4096, 1, 128, OP_C2C, SK_ROWS, -1, false, 2, 3, 9, 16, 16, 16)              \
     X(1, 4096, 1, 128, OP_C2C, SK_ROWS, 1, false, 2, 3, 9, 16, 16, 16)               \
     X(2, 2048, 1, 128, OP_C2C, SK_ROWS, -1, false, 2, 4, 9, 16, 16, 8)               \
     X(3, 2048, 1, 128, OP_C2C, SK_ROWS, 1, false, 2, 4, 9, 16, 16, 8)                \
-    X(4, 1024, 4, 256, OP_C2C, SK_ROWS, -1, false, 2, 2, 9, 16, 16, 4)               \
-    X(5, 1024, 4, 256, OP_C2C, SK_ROWS, 1, false, 2, 2, 9, 16, 16, 4)                \
+    X(4, 1024, 4, 128, OP_C2C, SK_ROWS, -1, false, 2, 3, 25, 32, 32)                \
+    X(5, 1024, 4, 128, OP_C2C, SK_ROWS, 1, false, 2, 3, 25, 32, 32)                 \
     /* rows of 256: 16 per 128-thread CTA with staged twiddles (the last    \
        axis of 256^3: 43.7 us against 48.5 with 8 per CTA, the variant) */   \
     X(6, 256, 16, 128, OP_C2C, SK_ROWS, -1, false, 2, 3, 11, 16, 16)                 \
     X(7, 256, 16, 128, OP_C2C, SK_ROWS, 1, false, 2, 3, 11, 16, 16)                  \
     X(6, 256, 8, 128, OP_C2C, SK_ROWS, -1, false, 2, 4, 9, 16, 16)                   \
     X(7, 256, 8, 128, OP_C2C, SK_ROWS, 1, false, 2, 4, 9, 16, 16)                    \
-    X(0, 8192, 1, 256, OP_C2C, SK_ROWS, -1, false, 2, 1, 9, 32, 16, 16)              \
-    X(1, 8192, 1, 256, OP_C2C, SK_ROWS, 1, false, 2, 1, 9, 32, 16, 16)               \
+    X(0, 8192, 1, 256, OP_C2C, SK_ROWS, -1, false, 2, 1, 27, 32, 16, 16)            \
+    X(1, 8192, 1, 256, OP_C2C, SK_ROWS, 1, false, 2, 1, 27, 32, 16, 16)             \
     /* strided axes of 2D / 3D transforms */                                  \
-    /* 2048-point columns: radix 32 first, 256 threads (200 us against 212 \
-       for 2048^2 x 8 with 16, 16, 8 on 512 threads, the hint variant) */    \
-    X(2, 2048, 8, 256, OP_C2C, SK_COLS, -1, false, 1, 1, 1, 32, 8, 8)                \
-    X(3, 2048, 8, 256, OP_C2C, SK_COLS, 1, false, 1, 1, 1, 32, 8, 8)                 \
+    /* 2048-point columns: in place, 4 columns per tile, so that the next   \
+       tile's input is staged meanwhile (176 us for 2048^2 x 8 against 193   \
+       with 8 columns and no room for it, a hint variant) */                 \
+    X(2, 2048, 4, 256, OP_C2C, SK_COLS, -1, false, 2, 1, 27, 16, 16, 8)             \
+    X(3, 2048, 4, 256, OP_C2C, SK_COLS, 1, false, 2, 1, 27, 16, 16, 8)              \
     X(2, 2048, 8, 512, OP_C2C, SK_COLS, -1, false, 1, 1, 1, 16, 16, 8)               \
     X(3, 2048, 8, 512, OP_C2C, SK_COLS, 1, false, 1, 1, 1, 16, 16, 8)                \
     /* 256-point column and transposed-row passes: 16 transforms per       \
@@ -70,21 +75,22 @@
        staged after it), keep the twiddles in shared memory (2) and, for     \
        R2C, run the last pass as mirrored butterfly pairs with the post-     \
        process fused (4); small CTAs (2-4 warps) leave more of them per SM.  \
+       C2R 6000 runs in place (251 us for 22369 rows against 278).            \
        The second entry of a length is a hint variant. */                    \
     X(0, 500, 2, 64, OP_R2C_HALF, SK_ROWS, -1, false, 2, 8, 15, 25, 5, 4)            \
     X(1, 500, 4, 128, OP_C2R_HALF, SK_ROWS, 1, false, 2, 4, 11, 20, 25)              \
     X(2, 3000, 1, 128, OP_R2C_HALF, SK_ROWS, -1, false, 2, 4, 15, 25, 15, 8)         \
-    X(3, 3000, 2, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 11, 25, 8, 15)          \
+    X(3, 3000, 1, 160, OP_C2R_HALF, SK_ROWS, 1, false, 2, 3, 27, 25, 12, 10)        \
     X(7, 3000, 1, 128, OP_C2R_HALF, SK_ROWS, 1, false, 2, 4, 9, 25, 8, 15)           \
     X(4, 3000, 1, 128, OP_R2C_HALF, SK_ROWS, -1, false, 2, 4, 7, 15, 25, 8)          \
     X(5, 3000, 2, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 1, 25, 8, 15)           \
     /* real rows of N = 2048, 4096, 8192 (half lengths 1024, 2048, 4096) */  \
-    X(6, 1024, 4, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 2, 15, 16, 16, 4)         \
-    X(7, 1024, 4, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 11, 16, 16, 4)          \
+    X(6, 1024, 4, 128, OP_R2C_HALF, SK_ROWS, -1, false, 2, 3, 31, 16, 16, 4)        \
+    X(7, 1024, 4, 128, OP_C2R_HALF, SK_ROWS, 1, false, 2, 3, 27, 32, 32)            \
     X(0, 2048, 1, 128, OP_R2C_HALF, SK_ROWS, -1, false, 2, 4, 15, 16, 16, 8)         \
     X(1, 2048, 1, 128, OP_C2R_HALF, SK_ROWS, 1, false, 2, 4, 15, 8, 16, 16)          \
-    X(2, 4096, 1, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 2, 15, 16, 32, 8)         \
-    X(3, 4096, 1, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 15, 16, 16, 16)         \
+    X(2, 4096, 1, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 2, 31, 16, 16, 16)       \
+    X(3, 4096, 1, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 25, 16, 16, 16)        \
     X(4, 1024, 4, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 3, 7, 16, 16, 4)          \
     X(5, 2048, 1, 128, OP_R2C_HALF, SK_ROWS, -1, false, 2, 4, 7, 16, 16, 8)          \
     X(6, 4096, 1, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 2, 7, 16, 32, 8)          \
@@ -94,12 +100,12 @@
     X(3, 50, 16, 128, OP_C2C, SK_ROWS, 1, false, 2, 4, 1, 5, 10)                     \
     X(4, 500, 10, 256, OP_C2C, SK_COLS, -1, false, 2, 2, 1, 25, 20)                  \
     X(5, 500, 10, 256, OP_C2C, SK_COLS, 1, false, 2, 2, 1, 25, 20)                   \
-    /* odd real length 2187 = 3^7, two rows per complex FFT (the R2C tile  \
-       shape from a run-time compiled sweep: 4 % faster than 2 x 192) */     \
-    X(7, 2187, 2, 128, OP_R2C_PAIR, SK_ROWS, -1, false, 2, 3, 15, 27, 9, 9)          \
-    /* C2R: one row pair per 128-thread CTA, four CTAs per SM (542 us for  \
-       122741 rows against 573 us with two pairs per 192-thread CTA) */      \
-    X(4, 2187, 1, 128, OP_C2R_PAIR, SK_ROWS, 1, false, 2, 4, 11, 27, 9, 9)           \
+    /* odd real length 2187 = 3^7, two rows per complex FFT, one row pair  \
+       per CTA, in place: R2C 260 us for 61370 rows against 283              \
+       self-sorting with two pairs */                                        \
+    X(7, 2187, 1, 128, OP_R2C_PAIR, SK_ROWS, -1, false, 2, 4, 31, 27, 9, 9)         \
+    /* C2R: 242 us against 261 self-sorting on 128 threads */              \
+    X(4, 2187, 1, 96, OP_C2R_PAIR, SK_ROWS, 1, false, 2, 5, 27, 27, 9, 9)           \
     X(0, 2187, 2, 192, OP_C2R_PAIR, SK_ROWS, 1, false, 2, 2, 11, 27, 9, 9)           \
     X(3, 2187, 2, 192, OP_C2R_PAIR, SK_ROWS, 1, false, 2, 2, 9, 27, 9, 9)            \
     X(1, 2187, 2, 128, OP_R2C_PAIR, SK_ROWS, -1, false, 2, 3, 1, 27, 9, 9)           \
@@ -134,9 +140,11 @@
     X(6, 256, 16, 256, OP_C2C, SK_COLS, -1, true, 2, 3, 9, 16, 16)                   \
     X(7, 256, 16, 256, OP_C2C, SK_COLS, 1, true, 2, 3, 9, 16, 16)                    \
     /* C2C 4096 rows, 256 threads per transform: taken automatically by row  \
-       steps of less than one wave of tiles (plan.cpp try_specialize) */     \
-    X(6, 4096, 1, 256, OP_C2C, SK_ROWS, -1, false, 2, 2, 9, 16, 16, 16)              \
-    X(7, 4096, 1, 256, OP_C2C, SK_ROWS, 1, false, 2, 2, 9, 16, 16, 16)               \
+       steps of less than one wave of tiles (plan.cpp try_specialize).  In    \
+       place straight from global memory: one tile per CTA has nothing to    \
+       stage ahead (4096 x 256: 5.1 us against 5.3 self-sorting) */          \
+    X(6, 4096, 1, 256, OP_C2C, SK_ROWS, -1, false, 1, 1, 17, 8, 32, 16)             \
+    X(7, 4096, 1, 256, OP_C2C, SK_ROWS, 1, false, 1, 1, 17, 8, 32, 16)              \
     X(0, 256, 16, 256, OP_C2C, SK_ROWS_T, -1, false, 2, 3, 9, 16, 16)                \
     X(1, 256, 16, 256, OP_C2C, SK_ROWS_T, 1, false, 2, 3, 9, 16, 16)                 \
     X(2, 256, 16, 256, OP_C2C, SK_COLS, -1, false, 2, 3, 9, 16, 16)                  \

@@ -41,76 +41,82 @@ SIP_HD constexpr int sk_pitch(int n, int r0) {
 
 // In-place layout (SK_IN_PLACE): the element with mixed-radix digits
 // d_0 .. d_{m-1} (n = d_0 N/R_0 + d_1 N/(R_0 R_1) + ...) of transform q lives at
-// slot sum d_i S_i of the transform: S_i = N/(R_0..R_i) for i > 0, and S_0 and the
-// pitch of the transforms padded by up to 15 slots.  Row tiles keep
-// transform q at q * pitch, column tiles interleave their P transforms
-// (slot * P + q).
+// slot sum d_i S_i of the transform, where S_{m-1} = 1, S_{m-2} is the last
+// radix plus up to 2 pad slots, the S_i between are the products of the radices
+// behind them, and S_0 and the pitch of the transforms are padded by up to
+// 15 slots.  Row tiles keep transform q at q * pitch, column tiles
+// interleave their P transforms (slot * P + q).
 //
-// The pads are chosen by counting: of the 16 candidates, the one whose passes
-// need the fewest shared-memory wavefronts (a wavefront serves 16 lanes in
-// 16 different 8-byte banks; lane order as in SkPass::butterfly_index).
+// The pads are chosen by counting: those whose passes need the fewest
+// shared-memory wavefronts (a wavefront serves 16 lanes in 16 different
+// 8-byte banks; lane order as in SkPass::butterfly_index), the smallest of
+// equal ones.
 struct SkIpLayout {
-    int s0, ld;
+    int pad, s0, ld;
 };
-SIP_HD constexpr int sk_ip_inner(const int* rs, int np, int i) {  // N / (R_0 .. R_i)
+// Stride of digit i > 0 (and the unpadded one of digit 0).
+SIP_HD constexpr int sk_ip_inner(const int* rs, int np, int i, int pad) {
     int s = 1;
-    for (int p = np - 1; p > i; --p) s *= rs[p];
+    for (int p = np - 1; p > i; --p) s *= rs[p] + (p == np - 1 ? pad : 0);
     return s;
 }
 // Slot of butterfly j of pass p.
-SIP_HD constexpr int sk_ip_slot_of(const int* rs, int np, int p, int s0, int j) {
-    int l = 1;
-    for (int i = 0; i < p; ++i) l *= rs[i];
-    const int m_count = sk_ip_inner(rs, np, p);
-    int k = p == np - 1 ? j : j / m_count, m = p == np - 1 ? 0 : j % m_count, s = 0;
+SIP_HD constexpr int sk_ip_slot_of(const int* rs, int np, int p, int pad, int s0, int j) {
+    int m_count = 1;
+    for (int i = p + 1; i < np; ++i) m_count *= rs[i];
+    int k = p == np - 1 ? j : j / m_count, s = 0;
+    const int m = p == np - 1 ? 0 : j % m_count;
     for (int i = 0; i < p; ++i) {
-        s += (k % rs[i]) * (i == 0 ? s0 : sk_ip_inner(rs, np, i));
+        s += (k % rs[i]) * (i == 0 ? s0 : sk_ip_inner(rs, np, i, pad));
         k /= rs[i];
     }
-    return s + m;
+    return s + m + (p < np - 2 ? m / rs[np - 1] * pad : 0);
 }
-SIP_HD constexpr int sk_ip_wavefronts(const int* rs, int np, int P, bool cols, bool cols_last, int s0, int ld) {
+SIP_HD constexpr int sk_ip_wavefronts(const int* rs, int np, int P, bool cols, bool cols_last, int pad, int s0,
+                                      int ld) {
     int n = 1, total = 0;
     for (int i = 0; i < np; ++i) n *= rs[i];
     for (int p = 0; p < np; ++p) {
         const int nr = n / rs[p];
         const bool q_first = cols || (cols_last && p == np - 1);
-        for (int h = 0; h < 6; ++h) {
+        for (int h = 0; h < 4; ++h) {
             int hit[16] = {}, worst = 0;
             for (int lane = 0; lane < 16; ++lane) {
                 const int b = h * 16 + lane;
                 if (b >= P * nr) break;
                 const int q = q_first ? b % P : b / nr, j = q_first ? b / P : b % nr;
-                const int slot = sk_ip_slot_of(rs, np, p, s0, j);
+                const int slot = sk_ip_slot_of(rs, np, p, pad, s0, j);
                 const int bank = (cols ? slot * P + q : q * ld + slot) % 16;
                 if (++hit[bank] > worst) worst = hit[bank];
             }
-            total += worst;
+            total += worst * (p == 0 || p == np - 1 ? 1 : 2);  // middle passes read and write
         }
     }
     return total;
 }
 SIP_HD constexpr SkIpLayout sk_ip_layout(const int* rs, int np, int P, bool cols, bool cols_last) {
-    const int base = sk_ip_inner(rs, np, 0);
-    SkIpLayout best{base, rs[0] * base};
+    SkIpLayout best{0, 0, 0};
     int cost = 1 << 30;
-    for (int pad = 0; pad < 16; ++pad) {
-        const int c = sk_ip_wavefronts(rs, np, 1, cols, false, base + pad, 0) +
-                      (cols ? sk_ip_wavefronts(rs, np, P, true, false, base + pad, 0) : 0);
-        if (c < cost) {
-            cost = c;
-            best.s0 = base + pad;
+    for (int pad = 0; pad < (np > 2 ? 3 : 1); ++pad) {
+        const int base = sk_ip_inner(rs, np, 0, pad);
+        for (int more = 0; more < 16; ++more) {
+            const int c = sk_ip_wavefronts(rs, np, cols ? P : 1, cols, false, pad, base + more, 0);
+            if (c < cost) {
+                cost = c;
+                best.pad = pad;
+                best.s0 = base + more;
+            }
         }
     }
     const int row = rs[0] * best.s0;
     best.ld = row;
     if (cols || P == 1) return best;
     cost = 1 << 30;
-    for (int pad = 0; pad < 16; ++pad) {
-        const int c = sk_ip_wavefronts(rs, np, P, false, cols_last, best.s0, row + pad);
+    for (int more = 0; more < 16; ++more) {
+        const int c = sk_ip_wavefronts(rs, np, P, false, cols_last, best.pad, best.s0, row + more);
         if (c < cost) {
             cost = c;
-            best.ld = row + pad;
+            best.ld = row + more;
         }
     }
     return best;
@@ -224,13 +230,24 @@ struct SkCfg {
     // the work layout is the only buffer; else the input is staged.
     static constexpr bool DIRECT = INPLACE && !SPLIT;
     static constexpr SkIpLayout LAY = INPLACE ? sk_ip_layout(rad_list, NP, P, MODE == SK_COLS, MODE == SK_ROWS_T)
-                                              : SkIpLayout{0, 0};
+                                              : SkIpLayout{0, 0, 0};
     static constexpr int LD = INPLACE ? LAY.ld : sk_pitch(N, radix(0));
     static constexpr int BUF = INPLACE ? sk_ip_buffer_values(P, LAY) : sk_buffer_values(OP, P, N, radix(0), FLAGS);
     static constexpr bool INTERLEAVED = INPLACE && MODE == SK_COLS;
     SIP_HD static constexpr int ip_at(int q, int s) { return INTERLEAVED ? s * P + q : q * LD + s; }
-    static constexpr int ip_stride(int p) { return p == 0 ? LAY.s0 : sk_ip_inner(rad_list, NP, p); }
-    static constexpr int ip_step(int p) { return ip_stride(p) * (INTERLEAVED ? P : 1); }
+    // (from scalars: a device function may not read the arrays and structs)
+    static constexpr int IP_PAD = LAY.pad, IP_S0 = LAY.s0;
+    SIP_HD static constexpr int ip_stride(int p) {
+        int st = 1;
+        for (int i = NP - 1; i > p; --i) st *= radix(i) + (i == NP - 1 ? IP_PAD : 0);
+        return p == 0 ? IP_S0 : st;
+    }
+    SIP_HD static constexpr int ip_step(int p) { return ip_stride(p) * (INTERLEAVED ? P : 1); }
+    // Slot of the digits after pass p, whose elements count m.
+    template <int PASS_>
+    SIP_HD static constexpr int ip_high(int m) {
+        return PASS_ < NP - 2 && IP_PAD > 0 ? m + m / radix(NP - 1) * IP_PAD : m;
+    }
     // Slot of the digits before pass p, whose transformed values count k < span(p).
     template <int PASS_>
     SIP_HD static constexpr int ip_low(int k) {
@@ -250,7 +267,7 @@ struct SkCfg {
         else return idx(u + r * (N / radix(NP - 1)));
     }
     SIP_HD static constexpr int first_slot(int u, int r) {
-        if constexpr (INPLACE) return u + r * ip_step(0);
+        if constexpr (INPLACE) return ip_high<0>(u) + r * ip_step(0);
         else return idx(u * radix(0) + r);
     }
     // Staged twiddles (SK_TW_SMEM): per pass p with span > 1, twcount rows
@@ -824,7 +841,7 @@ struct SkPass {
     SIP_HD static int ip_slot(int q, int j) {
         int k, m;
         split_index(j, k, m);
-        return K::ip_at(q, K::template ip_low<PASS>(k) + m);
+        return K::ip_at(q, K::template ip_low<PASS>(k) + K::template ip_high<PASS>(m));
     }
 
     SIP_HD static void butterfly_index(int b, int& q, int& j) {
@@ -2043,83 +2060,83 @@ __global__ void __launch_bounds__(K::T, K::MINB) sk_fft_kernel(const TileArgs a)
                 sk_ip_last<K>(tid, a, c, work);
             }
         }
-        return;
-    }
-    // staged twiddles after the buffers (the barrier before pass 0 of the
-    // first tile orders the copy before any use)
-    float2* tws = sk_smem + (STAGES == 2 ? 2 : 1) * K::BUF;
-    sk_load_tws<K>(tid, a, tws);
-    if constexpr (K::SPLIT) {
-        // buffers: bufs[0] stages the input, bufs[1] holds the work layout
-        static_assert(STAGES == 2, "a split pass 0 needs the staging and the work buffer");
-        sk_stage<K>(tid, a, decode_tile(a, tile), bufs[0]);
-        sk_commit();
-        for (; tile < a.ntiles; tile += gridDim.x) {
+    } else {
+        // staged twiddles after the buffers (the barrier before pass 0 of the
+        // first tile orders the copy before any use)
+        float2* tws = sk_smem + (STAGES == 2 ? 2 : 1) * K::BUF;
+        sk_load_tws<K>(tid, a, tws);
+        if constexpr (K::SPLIT) {
+            // buffers: bufs[0] stages the input, bufs[1] holds the work layout
+            static_assert(STAGES == 2, "a split pass 0 needs the staging and the work buffer");
+            sk_stage<K>(tid, a, decode_tile(a, tile), bufs[0]);
+            sk_commit();
+            for (; tile < a.ntiles; tile += gridDim.x) {
+                TileCtx c = decode_tile(a, tile);
+                c.tws = tws;
+                sk_wait<0>();
+                __syncthreads();
+                sk_load_cross<K>(tid, a, c, tws + K::TWSM);
+                if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
+                    sk_zero_missing<K>(tid, a, c, bufs[0]);
+                    __syncthreads();
+                }
+                sk_pass0_split<K>(tid, a, c, bufs[0], bufs[1]);
+                __syncthreads();
+                const int next = tile + gridDim.x;
+                if (next < a.ntiles) sk_stage<K>(tid, a, decode_tile(a, next), bufs[0]);
+                sk_commit();
+                sk_run<K, 1>(tid, a, c, bufs[1]);
+                if constexpr (sk_last_to_smem<K>()) sk_post<K>(tid, a, c, bufs[1]);
+                __syncthreads();
+            }
+            return;
+        }
+        if (STAGES == 2) {
+            sk_stage<K>(tid, a, decode_tile(a, tile), bufs[0]);
+            sk_commit();
+        }
+        for (int it = 0; tile < a.ntiles; ++it, tile += gridDim.x) {
+            float2* cur = bufs[it & 1];
             TileCtx c = decode_tile(a, tile);
             c.tws = tws;
-            sk_wait<0>();
+            if (STAGES == 2) {
+                const int next = tile + gridDim.x;
+                if (next < a.ntiles) sk_stage<K>(tid, a, decode_tile(a, next), bufs[(it + 1) & 1]);
+                sk_commit();
+                sk_wait<1>();
+            } else {
+                sk_stage<K>(tid, a, c, cur);
+                sk_commit();
+                sk_wait<0>();
+            }
             __syncthreads();
             sk_load_cross<K>(tid, a, c, tws + K::TWSM);
             if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
-                sk_zero_missing<K>(tid, a, c, bufs[0]);
+                sk_zero_missing<K>(tid, a, c, cur);
                 __syncthreads();
             }
-            sk_pass0_split<K>(tid, a, c, bufs[0], bufs[1]);
-            __syncthreads();
-            const int next = tile + gridDim.x;
-            if (next < a.ntiles) sk_stage<K>(tid, a, decode_tile(a, next), bufs[0]);
-            sk_commit();
-            sk_run<K, 1>(tid, a, c, bufs[1]);
-            if constexpr (sk_last_to_smem<K>()) sk_post<K>(tid, a, c, bufs[1]);
-            __syncthreads();
-        }
-        return;
-    }
-    if (STAGES == 2) {
-        sk_stage<K>(tid, a, decode_tile(a, tile), bufs[0]);
-        sk_commit();
-    }
-    for (int it = 0; tile < a.ntiles; ++it, tile += gridDim.x) {
-        float2* cur = bufs[it & 1];
-        TileCtx c = decode_tile(a, tile);
-        c.tws = tws;
-        if (STAGES == 2) {
-            const int next = tile + gridDim.x;
-            if (next < a.ntiles) sk_stage<K>(tid, a, decode_tile(a, next), bufs[(it + 1) & 1]);
-            sk_commit();
-            sk_wait<1>();
-        } else {
-            sk_stage<K>(tid, a, c, cur);
-            sk_commit();
-            sk_wait<0>();
-        }
-        __syncthreads();
-        sk_load_cross<K>(tid, a, c, tws + K::TWSM);
-        if constexpr (K::OP == OP_R2C_PAIR || K::OP == OP_C2R_PAIR) {
-            sk_zero_missing<K>(tid, a, c, cur);
+            if constexpr (K::OP == OP_PC) {
+                // forward FFT, filter, inverse FFT, all in shared memory.  The
+                // butterfly indices and addresses depend on the thread index
+                // alone; opaque copies of it per tile and half keep the
+                // compiler from hoisting them out of the tile loop (fewer
+                // spills: 240 against 328 bytes per thread for 4320 points as
+                // 18 x 16 x 15 on 288 threads)
+                int tid_fwd = tid;
+                asm volatile("" : "+r"(tid_fwd));
+                sk_half<SkView<K, OP_PC, -1, false>>(tid_fwd, a, c, cur);
+                sk_mul<K>(tid_fwd, a, c, cur);
+                __syncthreads();
+                int tid_inv = tid;
+                asm volatile("" : "+r"(tid_inv));
+                sk_half<SkView<K, OP_C2C, 1, true>>(tid_inv, a, c, cur);
+                __syncthreads();
+                continue;
+            }
+            sk_run<K, 0>(tid, a, c, cur);
+            if constexpr (sk_last_to_smem<K>()) sk_post<K>(tid, a, c, cur);
             __syncthreads();
         }
-        if constexpr (K::OP == OP_PC) {
-            // forward FFT, filter, inverse FFT, all in shared memory.  The
-            // butterfly indices and addresses depend on the thread index
-            // alone; opaque copies of it per tile and half keep the
-            // compiler from hoisting them out of the tile loop (fewer
-            // spills: 240 against 328 bytes per thread for 4320 points as
-            // 18 x 16 x 15 on 288 threads)
-            int tid_fwd = tid;
-            asm volatile("" : "+r"(tid_fwd));
-            sk_half<SkView<K, OP_PC, -1, false>>(tid_fwd, a, c, cur);
-            sk_mul<K>(tid_fwd, a, c, cur);
-            __syncthreads();
-            int tid_inv = tid;
-            asm volatile("" : "+r"(tid_inv));
-            sk_half<SkView<K, OP_C2C, 1, true>>(tid_inv, a, c, cur);
-            __syncthreads();
-            continue;
-        }
-        sk_run<K, 0>(tid, a, c, cur);
-        if constexpr (sk_last_to_smem<K>()) sk_post<K>(tid, a, c, cur);
-        __syncthreads();
     }
 }
 
