@@ -168,15 +168,14 @@ const std::vector<int>& tile_radices(int op, int n) {
 }
 
 // sk_ip_layout, searched once per radix order, tile and mode.
-SkIpLayout ip_layout(const std::vector<int>& radices, int P, int mode) {
+SkIpLayout ip_layout(const std::vector<int>& radices, int P, bool cols, bool cols_last) {
     static std::mutex& mu = *new std::mutex;
-    static auto& known = *new std::map<std::tuple<std::vector<int>, int, int>, SkIpLayout>;
-    const auto key = std::make_tuple(radices, P, mode);
+    static auto& known = *new std::map<std::tuple<std::vector<int>, int, bool, bool>, SkIpLayout>;
+    const auto key = std::make_tuple(radices, P, cols, cols_last);
     std::lock_guard<std::mutex> lk(mu);
     auto it = known.find(key);
     if (it == known.end())
-        it = known.emplace(key, sk_ip_layout(radices.data(), (int)radices.size(), P, mode == SK_COLS,
-                                             mode == SK_ROWS_T)).first;
+        it = known.emplace(key, sk_ip_layout(radices.data(), (int)radices.size(), P, cols, cols_last)).first;
     return it->second;
 }
 
@@ -351,7 +350,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     //    against 288; 945 135 against 128, 3375 150 against 141.
     const size_t passes = c.radices.size();
     int options = SK_TW_BASIS | SK_TW_SMEM | SK_SPLIT_PASS0;
-    if (op == OP_PC) options = SK_TW_BASIS | SK_IN_PLACE;
+    if (op == OP_PC) options |= SK_IN_PLACE;  // the staging only where it fits, below
     else if (op == OP_R2C_HALF || op == OP_R2C_PAIR) {
         if (passes >= 3 || c.radices.back() <= 21) options |= SK_IN_PLACE | SK_MIRROR_PAIR;
     } else if (passes >= 3 && (op != OP_C2R_PAIR || n > 5000)) options |= SK_IN_PLACE;
@@ -372,7 +371,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
         const int* rs = c.radices.data();
         Bytes s{};
         if (inplace) {
-            *lay = ip_layout(c.radices, P, mode);
+            *lay = ip_layout(c.radices, P, mode == SK_COLS, mode == SK_ROWS_T || sk_pulse_cols(op, tw4, options));
             s.buf = 8LL * sk_ip_buffer_values(P, *lay);
             s.staged = (options & SK_SPLIT_PASS0) ? 8LL * ((sk_stage_slots(op, P, n, options) + 1) / 2 * 2) : 0;
         } else {
@@ -384,6 +383,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
         return s;
     };
     SkIpLayout lay{0, 0, 0};
+    auto ctas = [](long long b) { return (int)std::max(1LL, (228 * 1024) / (b + 1024)); };
 
     // transforms per tile: about SIP_FFT_JIT_TILE (4096) values for rows, runs
     // of 16 adjacent transforms (128-byte segments) for the column modes, 8 or
@@ -391,7 +391,9 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     // values in columns of 1000: 140 us with 8, 203 with 16 and no room;
     // 2048: 176 us with 4, 193 with 8); at most SIP_FFT_JIT_E (32) values
     // per thread and pass
-    const int tile_values = std::max(64, env_int("SIP_FFT_JIT_TILE", 4096));
+    // Pulse rows: 2900, so that four CTAs stage their input (rows of 720 53 us
+    // for 8.4 M values against 60, Bluestein's 509 x 16502 99 against 134).
+    const int tile_values = std::max(64, env_int("SIP_FFT_JIT_TILE", op == OP_PC && !tw4 ? 2900 : 4096));
     const int per_thread = std::max(8, values > 0 ? values : env_int("SIP_FFT_JIT_E", 32));
     long long P = std::max(1, tile_values / n);
     if (mode != SK_ROWS) {
@@ -417,10 +419,16 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     if (ovr_int("SIP_FFT_JIT_T", 0) > 0) T = ovr_int("SIP_FFT_JIT_T", 0);
     if (T % 32 != 0 || T > kMaxTileThreads) return false;
     c.P = (int)P;
+    if (op == OP_PC && inplace && ovr_int("SIP_FFT_JIT_TWB", -1) < 0) {
+        // Pulse tiles stage their input and twiddles where four CTAs of them
+        // still fit an SM (2304: 54 us for 8.4 M values against 66), else they
+        // read global memory directly (4096: 52 against 61, 8820: 79 against 97).
+        const Bytes all = bytes(c.P, &lay);
+        if (ctas(all.buf + all.staged + all.cross + all.tws) < 4) options &= ~(SK_SPLIT_PASS0 | SK_TW_SMEM);
+    }
     c.twb = options;
     const Bytes s = bytes(c.P, &lay);
     c.LD = inplace ? lay.ld : sk_pitch(n, c.radices[0]);
-    auto ctas = [](long long b) { return (int)std::max(1LL, (228 * 1024) / (b + 1024)); };
     // The staged twiddles give way to the staged input, and to a second CTA
     // per SM (C2C rows of 7000: 146 us with two CTAs of 256 threads and the
     // twiddles through L1, 154 with one of 352).
@@ -451,7 +459,7 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
         // threads, 251 with 2 of 256, 328 with 1 of 288; 8640: 248 us with 2 of
         // 256, 326 with 1 of 384.  `values` other than 32: half the CTAs, for
         // tiles that spill.
-        const int fit = ctas(s.buf + tws);
+        const int fit = ctas(c.smem);
         c.T = fit >= 4 ? 128 : fit >= 2 ? 256 : 512;
         c.minb = std::max(1, std::min(fit, 512 / c.T) / (per_thread == 32 ? 1 : 2));
         if (ovr_int("SIP_FFT_JIT_T", 0) > 0) c.T = ovr_int("SIP_FFT_JIT_T", 0);

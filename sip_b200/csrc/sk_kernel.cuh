@@ -121,6 +121,10 @@ SIP_HD constexpr SkIpLayout sk_ip_layout(const int* rs, int np, int P, bool cols
     }
     return best;
 }
+// Four-step pulse tiles in place: the last forward pass runs lanes along rows.
+SIP_HD constexpr bool sk_pulse_cols(int op, bool tw4, int flags) {
+    return op == OP_PC && tw4 && (flags & SK_IN_PLACE) != 0;
+}
 SIP_HD constexpr int sk_ip_buffer_values(int p, SkIpLayout lay) { return (p * lay.ld + 1) / 2 * 2; }
 
 SIP_HD constexpr int sk_twcount(int r, bool basis) { return basis ? basis_count(r) : r - 1; }
@@ -215,8 +219,13 @@ struct SkCfg {
     }
     static constexpr int tw_entries() { return twoff(NP); }
     static constexpr int idx(int n) { return sk_index(n, radix(0)); }
+    // Lanes of pass p run along the transforms: column tiles, the pass that
+    // stores adjacent columns, and the last forward pass of a four-step
+    // pulse tile, whose filter values of adjacent rows are adjacent (lanes
+    // along k read one 32-byte sector each for 8 bytes: 131 us against 84 for
+    // the row pass of 65536 x 256).
     static constexpr bool colmap(int p) {
-        return MODE == SK_COLS || (MODE == SK_ROWS_T && p == NP - 1 && OP == OP_C2C);
+        return MODE == SK_COLS || (p == NP - 1 && ((MODE == SK_ROWS_T && OP == OP_C2C) || sk_pulse_cols(OP, TW4, FLAGS)));
     }
     // Mirrored-tile ops: slots [0, H) hold rows / columns c*H + q of the first
     // half, slots [H, 2H) their mirrors (sk_mirror_*).
@@ -229,8 +238,9 @@ struct SkCfg {
     // In-place layout (sk_ip_layout).  DIRECT: pass 0 reads global memory and
     // the work layout is the only buffer; else the input is staged.
     static constexpr bool DIRECT = INPLACE && !SPLIT;
-    static constexpr SkIpLayout LAY = INPLACE ? sk_ip_layout(rad_list, NP, P, MODE == SK_COLS, MODE == SK_ROWS_T)
-                                              : SkIpLayout{0, 0, 0};
+    static constexpr SkIpLayout LAY =
+        INPLACE ? sk_ip_layout(rad_list, NP, P, MODE == SK_COLS, MODE == SK_ROWS_T || sk_pulse_cols(OP, TW4, FLAGS))
+                : SkIpLayout{0, 0, 0};
     static constexpr int LD = INPLACE ? LAY.ld : sk_pitch(N, radix(0));
     static constexpr int BUF = INPLACE ? sk_ip_buffer_values(P, LAY) : sk_buffer_values(OP, P, N, radix(0), FLAGS);
     static constexpr bool INTERLEAVED = INPLACE && MODE == SK_COLS;
