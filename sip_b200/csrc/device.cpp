@@ -198,6 +198,20 @@ ChunkLanes::~ChunkLanes() {
     if (side) cudaStreamDestroy(side);
 }
 
+namespace {
+
+// A second lane, or null where the device has none left.
+std::shared_ptr<ChunkLanes> make_lanes() {
+    auto l = std::make_shared<ChunkLanes>();
+    if (cudaStreamCreateWithFlags(&l->side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&l->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&l->join, cudaEventDisableTiming) != cudaSuccess)
+        return nullptr;
+    return l;
+}
+
+}  // namespace
+
 void prepare_device(FftPlan& plan) {
     int device = -1;
     check(cudaGetDevice(&device), "cudaGetDevice");
@@ -207,13 +221,13 @@ void prepare_device(FftPlan& plan) {
     // serving loop's plain path) would pay every time.  A plan without it
     // runs its chunks on one lane.
     bool chunked = false;
-    for (const ChunkGroup& g : plan.chunk_groups) chunked = chunked || chunk_units(g) < g.units;
+    // The groups of size_default_chunks get it with their plan's second exec
+    // (launch_steps): a plan that runs once does not pay for it at all.
+    for (const ChunkGroup& g : plan.chunk_groups)
+        chunked = chunked || (!chunks_by_default(g) && chunk_units(g) < g.units);
     if (chunked) {
-        auto l = std::make_shared<ChunkLanes>();
-        check(cudaStreamCreateWithFlags(&l->side, cudaStreamNonBlocking), "cudaStreamCreate");
-        check(cudaEventCreateWithFlags(&l->fork, cudaEventDisableTiming), "cudaEventCreate");
-        check(cudaEventCreateWithFlags(&l->join, cudaEventDisableTiming), "cudaEventCreate");
-        plan.lanes = l;
+        plan.lanes = make_lanes();
+        if (plan.lanes == nullptr) check(cudaGetLastError(), "chunk lanes");
     }
     for (Step& st : plan.steps) {
         if (is_pair_kind(st.kind)) continue;  // no tables
@@ -372,14 +386,26 @@ void launch_rows(const FftPlan& plan, long long rows, const void* in, void* out,
 // group are reused by every chunk, so the intermediate one step writes and
 // the next reads stays in L2 and the chain costs about one HBM round trip
 // of its input and output instead of one per step.
-void launch_steps(const FftPlan& plan, const void* in, void* out, void* ws) {
+void launch_steps(const FftPlan& plan, const void* in, void* out, void* ws, bool may_allocate) {
     cudaStream_t stream = static_cast<cudaStream_t>(plan.stream);
+    // The second lane of default chunks, made with the second exec (not while
+    // the stream is being captured, and not by an exec that may not allocate);
+    // without it those groups run as whole passes.
+    bool wants_lane = false;
+    for (const ChunkGroup& g : plan.chunk_groups) wants_lane = wants_lane || chunks_by_default(g);
+    if (wants_lane && plan.lanes == nullptr && chunk_lanes() == 2 && may_allocate && plan.ran) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
+            plan.lanes = make_lanes();
+        if (plan.lanes == nullptr) (void)cudaGetLastError();
+    }
+    plan.ran = true;
     for (size_t i = 0; i < plan.steps.size();) {
         const int gi = plan.steps[i].chunk_group;
         if (gi >= 0) {
             const ChunkGroup& g = plan.chunk_groups[gi];
             const long long cu = chunk_units(g);
-            if (cu < g.units) {
+            if (cu < g.units && (!chunks_by_default(g) || plan.lanes != nullptr)) {
                 // lane 0 is the plan's stream; lane 1 forks from it and joins
                 // it again after the group
                 const bool two = plan.lanes != nullptr && chunk_lanes() == 2;

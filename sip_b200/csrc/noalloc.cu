@@ -69,7 +69,7 @@ int noalloc_exec(const FftPlan& p, const void* in, void* out) {
         return kNaInternal;
     }
     try {
-        launch_steps(p, in, out, p.noalloc_scratch);
+        launch_steps(p, in, out, p.noalloc_scratch, false);
     } catch (const std::exception& ex) {
         std::fprintf(stderr, "[sip_b200] no-alloc exec failed: %s\n", ex.what());
         return kNaInternal;

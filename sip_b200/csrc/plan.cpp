@@ -1243,6 +1243,28 @@ bool make_chunk_group(FftPlan& plan, size_t first, size_t last, long long units)
     return true;
 }
 
+bool chunk_requested() {
+    const char* req = std::getenv("SIP_FFT_L2_CHUNK_MB");
+    return g_chunk_override.load() >= 0 || (req != nullptr && *req != '\0');
+}
+
+// Multi-D C2C plans whose passes run faster chunk by chunk.  3-D from 48 MB of
+// data: 256^3 122 us in chunks of 32 MB against 138 whole, 64^3 x 64 107
+// against 145, 98 x 128 x 147 x 4 71 against 82.  2-D from 64 MB, where an
+// item is small enough for the chunk's passes to fill whole waves (512^2 x 64
+// 88 against 103 us, 256^2 x 512 153 against 193) or a chunk by itself
+// (2048^2 x 4 130 against 137); between them it loses up to 5 % (1000^2 x 33,
+// 450 x 1280 x 58).  Real multi-D plans gain in some shapes and lose in others
+// (0.9-1.2x), so they stay whole.
+bool multid_chunks_pay(const FftPlan& plan, long long item) {
+    if (plan.type != ASCEND_FFT_C2C || plan.out_shift != 0 || plan.hint_generic) return false;
+    for (const Step& st : plan.steps)
+        if (st.kind != StepKind::Tile) return false;
+    const long long total = item * plan.batch;
+    if (plan.sizes.size() == 3) return total >= (48LL << 20);
+    return total >= (64LL << 20) && (item <= (2LL << 20) || item >= (24LL << 20));
+}
+
 // Chunk groups of a built plan.  1-D plans (and pulse plans): every step
 // carries the batch rows, so the whole chain runs row chunk by row chunk.
 // Multi-D plans: whole batch items per chunk when an item fits the chunk
@@ -1266,14 +1288,13 @@ void form_chunk_groups(FftPlan& plan) {
         make_chunk_group(plan, 0, ns, plan.batch);
         return;
     }
-    // Multi-D chunks only on request (SIP_FFT_L2_CHUNK_MB or the test hook):
-    // measured slower than the unchunked axis passes on B200 (2048^2 x 8:
-    // 0.34 ms unchunked, 0.38-0.40 ms in chunks of one or two items).
-    const char* req = std::getenv("SIP_FFT_L2_CHUNK_MB");
-    if (g_chunk_override.load() < 0 && (req == nullptr || *req == '\0')) return;
     long long item = 8;
     for (int64_t s : plan.sizes) item *= s;
-    const long long target = chunk_target_bytes();
+    // Without a request (SIP_FFT_L2_CHUNK_MB or the test hook) multi-D plans
+    // are grouped for the chunks of size_default_chunks only.
+    const bool requested = chunk_requested();
+    if (!requested && !multid_chunks_pay(plan, item)) return;
+    const long long target = requested ? chunk_target_bytes() : std::max(kL2ChunkBytes, plan.sizes.size() == 2 ? item : 0LL);
     if (target > 0 && item <= target) {
         make_chunk_group(plan, 0, ns, plan.batch);
         return;
@@ -1289,6 +1310,31 @@ void form_chunk_groups(FftPlan& plan) {
         if (!make_chunk_group(plan, 0, 2, plan.batch * X)) {
             s0.chunk_per = p0;
             s1.chunk_per = p1;
+        }
+    }
+}
+
+// Chunk sizes used without a request, for the groups that two lanes of
+// L2-sized chunks run faster than whole passes: what one pass writes, the
+// next one reads from L2, and the second lane fills the first one's partial
+// waves.  1-D and pulse chains of tile steps from 64 MB of data, in chunks of
+// half the data but at most 96 MB: C2C 65536 x 4096 1.36 ms against 1.50,
+// pulse 65536 x 256 170 us against 190, R2C 2^20 x 256 1.06 ms against 1.19; no
+// C2C, R2C or pulse shape of 2^15 to 2^20 points measured slower.  Chains
+// with an element-wise real pass do (C2R 2^20 x 256: 1.28 ms against 1.23).
+// Units of 16 MB and more keep the chunks of chunk_units.
+void size_default_chunks(FftPlan& plan) {
+    if (chunk_requested() || plan.hint_generic || plan.out_shift != 0) return;
+    for (ChunkGroup& g : plan.chunk_groups) {
+        const long long total = g.units * g.unit_bytes;
+        bool tiles = true;
+        for (size_t i = g.first; i < g.last; ++i) tiles = tiles && plan.steps[i].kind == StepKind::Tile;
+        if (!tiles || plan.compute_mode != kComputeFp32) continue;
+        if (plan.sizes.size() == 1 || plan.pulse) {
+            if (total >= (64LL << 20) && g.unit_bytes < kL2ChunkMinUnit)
+                g.target = std::min(96LL << 20, std::max(kL2ChunkBytes, total / 2));
+        } else {
+            g.target = std::max(kL2ChunkBytes, g.unit_bytes);
         }
     }
 }
@@ -1329,7 +1375,10 @@ long long chunk_min_unit_bytes() {
     return v;
 }
 
+bool chunks_by_default(const ChunkGroup& g) { return g.target > 0 && !chunk_requested(); }
+
 long long chunk_units(const ChunkGroup& g) {
+    if (chunks_by_default(g)) return std::max(1LL, std::min(g.units, g.target / std::max(1LL, g.unit_bytes)));
     const long long target = chunk_target_bytes();
     if (target <= 0 || g.unit_bytes <= 0 || g.unit_bytes < chunk_min_unit_bytes()) return g.units;
     return std::max(1LL, std::min(g.units, target / g.unit_bytes));
@@ -1385,6 +1434,7 @@ TileLaunch chunk_tile_launch(const Step& st, long long cnt) {
 void build_steps(FftPlan& plan) {
     build_steps_inner(plan);
     form_chunk_groups(plan);
+    size_default_chunks(plan);
 }
 
 namespace {

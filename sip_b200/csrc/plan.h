@@ -130,6 +130,7 @@ struct ChunkGroup {
     size_t first = 0, last = 0;
     long long units = 0;
     long long unit_bytes = 0;
+    long long target = 0;  // chunk bytes without a request (plan.cpp size_default_chunks; 0: chunk_units' defaults)
 };
 
 struct FftPlan {
@@ -172,7 +173,8 @@ struct FftPlan {
     std::vector<ChunkGroup> chunk_groups;
     // Second stream and fork / join events of the two chunk lanes (made at
     // device preparation when the plan has chunk groups).
-    std::shared_ptr<ChunkLanes> lanes;
+    mutable std::shared_ptr<ChunkLanes> lanes;
+    mutable bool ran = false;  // an exec was launched (launch_steps)
 
     bool forward() const { return direction == AsdSip::ASCEND_FFT_FORWARD; }
     int64_t elements() const;  // batch * prod(sizes)
@@ -226,7 +228,8 @@ int batch_last_launches(const Batch* b);
 void launch_separated(const FftPlan& plan, const float* in_re, const float* in_im, float* out_re, float* out_im);
 
 // Launches every step on the plan's stream (chunk groups chunk by chunk).
-void launch_steps(const FftPlan& plan, const void* in, void* out, void* ws);
+// `may_allocate` false: no stream or event is made for them.
+void launch_steps(const FftPlan& plan, const void* in, void* out, void* ws, bool may_allocate = true);
 
 // True when every step of the plan can run on the first rows of its batch
 // alone (1-D and pulse plans of tile and real pre/post steps).
@@ -239,6 +242,8 @@ void launch_rows(const FftPlan& plan, long long rows, const void* in, void* out,
 // (SIP_FFT_L2_CHUNK_MB, default kL2ChunkBytes; 0 turns chunking off); the
 // group's `units` when it runs as one launch per step.
 long long chunk_units(const ChunkGroup& g);
+// The group runs in the chunks of size_default_chunks (no request).
+bool chunks_by_default(const ChunkGroup& g);
 constexpr long long kL2ChunkBytes = 32LL << 20;
 // Units smaller than this run unchunked (plan.cpp chunk_min_unit_bytes).
 constexpr long long kL2ChunkMinUnit = 16LL << 20;
