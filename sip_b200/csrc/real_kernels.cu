@@ -12,45 +12,102 @@ namespace sipfft {
 
 namespace {
 
-// One thread per pair (k, m - k), k in [0, m/2]: each value and each
-// twiddle is read once (the mirror's twiddle follows from W_{2m}^k).
+// One thread per pair (k, m - k), k in [0, m/2], of kRealRows rows: each value
+// is read once, the mirror's twiddle follows from W_{2m}^k, and the rows share
+// the twiddle (a third of the loads otherwise, from a table of 8 m bytes) and
+// have their loads in flight together.  C2R 2^20 x 256: 319 us for the
+// pre-process (6.7 TB/s) against 449 with one row per thread.  Passes of less
+// than a GPU full of such threads take one row per thread, for the threads.
+constexpr int kRealRowsMany = 4;
+constexpr long long kRealRowsMin = 4LL * 148 * 2048;  // pairs of all rows
+
+template <int kRealRows>
 __global__ void k_real_post(const RealPassArgs a) {
     grid_dep_wait();
     grid_dep_launch();
     const long long pairs = a.m / 2 + 1;
     const bool cj = a.conj != 0;
-    for (long long row = blockIdx.y; row < a.rows; row += gridDim.y) {
+    for (long long row = (long long)kRealRows * blockIdx.y; row < a.rows; row += (long long)kRealRows * gridDim.y) {
+        const int cnt = (int)(a.rows - row < kRealRows ? a.rows - row : kRealRows);
         const float2* z = a.src + row * a.in_pitch;
         float2* x = a.dst + row * a.out_pitch;
         for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < pairs;
              k += (long long)gridDim.x * blockDim.x) {
             const long long km = a.m - k;
-            if (k > 0 && k < km) {
-                real_post_pair(z, k, a.m, a.tw, cj, x + k, x + km);
-            } else {
-                x[k] = real_post_elem(z, k, a.m, a.tw, cj);
-                if (km != k) x[km] = real_post_elem(z, km, a.m, a.tw, cj);
+            if (cnt == kRealRows && k > 0 && k < km) {
+                const float2 w = __ldg(a.tw + k);
+                float2 u[kRealRows], v[kRealRows];
+#pragma unroll
+                for (int r = 0; r < kRealRows; ++r) {
+                    u[r] = __ldg(z + r * a.in_pitch + k);
+                    v[r] = __ldg(z + r * a.in_pitch + km);
+                }
+#pragma unroll
+                for (int r = 0; r < kRealRows; ++r) {  // real_post_pair
+                    const float2 ev = make_float2(0.5f * (u[r].x + v[r].x), 0.5f * (u[r].y - v[r].y));
+                    const float2 od = make_float2(0.5f * (u[r].y + v[r].y), -0.5f * (u[r].x - v[r].x));
+                    const float2 t = c_mul(w, od);
+                    const float2 p = c_add(ev, t), q = make_float2(ev.x - t.x, t.y - ev.y);
+                    x[r * a.out_pitch + k] = cj ? c_conj(p) : p;
+                    x[r * a.out_pitch + km] = cj ? c_conj(q) : q;
+                }
+                continue;
+            }
+            for (int r = 0; r < cnt; ++r) {
+                const float2* zr = z + r * a.in_pitch;
+                float2* xr = x + r * a.out_pitch;
+                if (k > 0 && k < km) {
+                    real_post_pair(zr, k, a.m, a.tw, cj, xr + k, xr + km);
+                } else {
+                    xr[k] = real_post_elem(zr, k, a.m, a.tw, cj);
+                    if (km != k) xr[km] = real_post_elem(zr, km, a.m, a.tw, cj);
+                }
             }
         }
     }
 }
 
+template <int kRealRows>
 __global__ void k_real_pre(const RealPassArgs a) {
     grid_dep_wait();
     grid_dep_launch();
     const long long pairs = a.m / 2 + 1;
     const bool cj = a.conj != 0;
-    for (long long row = blockIdx.y; row < a.rows; row += gridDim.y) {
+    const float sg = cj ? -0.5f : 0.5f;
+    for (long long row = (long long)kRealRows * blockIdx.y; row < a.rows; row += (long long)kRealRows * gridDim.y) {
+        const int cnt = (int)(a.rows - row < kRealRows ? a.rows - row : kRealRows);
         const float2* x = a.src + row * a.in_pitch;
         float2* z = a.dst + row * a.out_pitch;
         for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < pairs;
              k += (long long)gridDim.x * blockDim.x) {
             const long long km = a.m - k;
-            if (k > 0 && k < km) {
-                real_pre_pair(x, k, a.m, a.tw, cj, z + k, z + km);
-            } else {
-                z[k] = real_pre_elem(x, k, a.m, a.tw, cj);
-                if (km != k && km < a.m) z[km] = real_pre_elem(x, km, a.m, a.tw, cj);
+            if (cnt == kRealRows && k > 0 && k < km) {
+                const float2 w = __ldg(a.tw + k);
+                float2 u[kRealRows], v[kRealRows];
+#pragma unroll
+                for (int r = 0; r < kRealRows; ++r) {
+                    u[r] = __ldg(x + r * a.in_pitch + k);
+                    v[r] = __ldg(x + r * a.in_pitch + km);
+                }
+#pragma unroll
+                for (int r = 0; r < kRealRows; ++r) {  // real_pre_pair
+                    const float2 e = make_float2(0.5f * (u[r].x + v[r].x), sg * (u[r].y - v[r].y));
+                    const float2 d = make_float2(0.5f * (u[r].x - v[r].x), sg * (u[r].y + v[r].y));
+                    const float2 od = c_mulc(d, w);
+                    z[r * a.out_pitch + k] = make_float2(e.x - od.y, e.y + od.x);
+                    z[r * a.out_pitch + km] = make_float2(e.x + od.y, od.x - e.y);
+                }
+                continue;
+            }
+            for (int r = 0; r < cnt; ++r) {
+                const float2* xr = x + r * a.in_pitch;
+                float2* zr = z + r * a.out_pitch;
+                if (k > 0 && k < km) {
+                    real_pre_pair(xr, k, a.m, a.tw, cj, zr + k, zr + km);
+                } else {
+                    zr[k] = real_pre_elem(xr, k, a.m, a.tw, cj);
+                    if (km != k && km < a.m) zr[km] = real_pre_elem(xr, km, a.m, a.tw, cj);
+                }
             }
         }
     }
@@ -131,11 +188,19 @@ dim3 grid_for(long long per_row, long long rows, int block) {
 }  // namespace
 
 cudaError_t real_post(const RealPassArgs& a, cudaStream_t stream) {
-    return launch_pdl(k_real_post, grid_for(a.m / 2 + 1, a.rows, 256), dim3(256), 0, stream, a.m * a.rows, a);
+    const long long pairs = a.m / 2 + 1;
+    if (pairs * a.rows < kRealRowsMin)
+        return launch_pdl(k_real_post<1>, grid_for(pairs, a.rows, 256), dim3(256), 0, stream, a.m * a.rows, a);
+    return launch_pdl(k_real_post<kRealRowsMany>, grid_for(pairs, (a.rows + kRealRowsMany - 1) / kRealRowsMany, 256),
+                      dim3(256), 0, stream, a.m * a.rows, a);
 }
 
 cudaError_t real_pre(const RealPassArgs& a, cudaStream_t stream) {
-    return launch_pdl(k_real_pre, grid_for(a.m / 2 + 1, a.rows, 256), dim3(256), 0, stream, a.m * a.rows, a);
+    const long long pairs = a.m / 2 + 1;
+    if (pairs * a.rows < kRealRowsMin)
+        return launch_pdl(k_real_pre<1>, grid_for(pairs, a.rows, 256), dim3(256), 0, stream, a.m * a.rows, a);
+    return launch_pdl(k_real_pre<kRealRowsMany>, grid_for(pairs, (a.rows + kRealRowsMany - 1) / kRealRowsMany, 256),
+                      dim3(256), 0, stream, a.m * a.rows, a);
 }
 
 cudaError_t pair_pack(const PairPassArgs& a, cudaStream_t stream) {

@@ -60,9 +60,9 @@
     /* four-step 2^19 = 512 x 1024 (real 2^20) */                             \
     /* 8 columns per 128-thread CTA, staged twiddles, split pass 0 (C2R    \
        2^20 x 256 pass A: 585 us against 602 with 16 per 256-thread CTA) */  \
-    X(2, 512, 8, 128, OP_C2C, SK_COLS, -1, true, 2, 3, 11, 16, 32)                   \
+    X(2, 512, 8, 128, OP_C2C, SK_COLS, -1, true, 2, 3, 11, 32, 16)                  \
     X(2, 512, 16, 256, OP_C2C, SK_COLS, -1, true, 1, 3, 1, 16, 32)                   \
-    X(3, 512, 8, 128, OP_C2C, SK_COLS, 1, true, 2, 3, 11, 16, 32)                    \
+    X(3, 512, 8, 128, OP_C2C, SK_COLS, 1, true, 2, 3, 11, 32, 16)                   \
     X(3, 512, 16, 256, OP_C2C, SK_COLS, 1, true, 1, 3, 1, 16, 32)                    \
     /* pass B on rows of 1024: staged twiddles, split pass 0, double       \
        buffer (C2R 2^20 x 256: 409 us against 435 single-buffered) */        \
@@ -119,13 +119,15 @@
     X(0, 1024, 8, 256, OP_R2C_4B, SK_ROWS_T, -1, false, 1, 2, 3, 32, 32)             \
     /* the split 2^19 = 1024 x 512: columns of 1024 (pass A), R2C pass B +  \
        post on rows of 512, C2C pass B on rows of 512 */                     \
-    X(6, 1024, 8, 256, OP_C2C, SK_COLS, -1, true, 1, 3, 1, 32, 32)                   \
-    X(7, 1024, 8, 256, OP_C2C, SK_COLS, 1, true, 1, 3, 1, 32, 32)                    \
+    X(6, 1024, 8, 256, OP_C2C, SK_COLS, -1, true, 2, 1, 27, 32, 32)                 \
+    X(7, 1024, 8, 256, OP_C2C, SK_COLS, 1, true, 2, 1, 27, 32, 32)                  \
     X(2, 512, 16, 256, OP_R2C_4B, SK_ROWS_T, -1, false, 1, 2, 1, 16, 32)             \
     X(3, 512, 16, 256, OP_R2C_4B, SK_ROWS_T, -1, false, 2, 1, 1, 16, 32)             \
-    /* R2C pass B with the post-process on mirrored butterfly pairs (TWB 5): \
-       rows of 512 (split 1024 x 512) and of 1024 (split 512 x 1024) */      \
-    X(4, 512, 16, 256, OP_R2C_4B, SK_ROWS_T, -1, false, 1, 2, 5, 32, 16)             \
+    /* R2C pass B with the post-process on mirrored butterfly pairs: rows of  \
+       512 (split 1024 x 512; in place with the next tile's rows staged, R2C  \
+       2^20 x 256 in whole passes 1.02 ms against 1.19 self-sorting from one  \
+       buffer) and of 1024 (split 512 x 1024) */                              \
+    X(4, 512, 16, 256, OP_R2C_4B, SK_ROWS_T, -1, false, 2, 1, 31, 32, 16)           \
     X(5, 1024, 16, 512, OP_R2C_4B, SK_ROWS_T, -1, false, 1, 1, 5, 16, 4, 16)         \
     /* C2R pre-process + pass A on mirrored butterfly pairs (TWB 5) */       \
     X(6, 512, 16, 256, OP_C2R_4A, SK_COLS, 1, false, 1, 2, 5, 16, 32)                \

@@ -239,7 +239,7 @@ struct SkCfg {
     // the work layout is the only buffer; else the input is staged.
     static constexpr bool DIRECT = INPLACE && !SPLIT;
     static constexpr SkIpLayout LAY =
-        INPLACE ? sk_ip_layout(rad_list, NP, P, MODE == SK_COLS, MODE == SK_ROWS_T || sk_pulse_cols(OP, TW4, FLAGS))
+        INPLACE ? sk_ip_layout(rad_list, NP, MIRROR ? P / 2 : P, MODE == SK_COLS, MODE == SK_ROWS_T || sk_pulse_cols(OP, TW4, FLAGS))
                 : SkIpLayout{0, 0, 0};
     static constexpr int LD = INPLACE ? LAY.ld : sk_pitch(N, radix(0));
     static constexpr int BUF = INPLACE ? sk_ip_buffer_values(P, LAY) : sk_buffer_values(OP, P, N, radix(0), FLAGS);
@@ -328,7 +328,8 @@ struct SkCfg {
     static_assert(!MPAIR || (OP != OP_C2R_HALF && OP != OP_C2R_PAIR) || SIGN > 0,
                   "C2R tiles run the inverse transform");
     static_assert(!SPLIT || (NP >= 2 && (OP != OP_PC || INPLACE)), "a split pass 0 needs a later pass, and no pulse tile");
-    static_assert(!INPLACE || (NP >= 2 && OP != OP_C2R_4A && OP != OP_R2C_4B), "in-place tiles: two or more passes");
+    static_assert(!INPLACE || (NP >= 2 && OP != OP_C2R_4A && (OP != OP_R2C_4B || (SPLIT && MPAIR))),
+                  "in-place tiles: two or more passes; mirrored rows staged and on pairs");
     static_assert(TWSM == sk_tws_values(OP_, N_, rad_list, NP, TWB_), "staged twiddle layout");
 };
 
@@ -581,6 +582,21 @@ SIP_HD void sk_stage(int tid, const TileArgs& a, const TileCtx& c, float2* stage
         // rows k1 = i0 + q (slot q) and N1 - k1 (slot H + q) of Y, N values each
         const int n1 = a.n_other;
         const char* ybase = src + (c.in_base - (long long)c.i0 * K::N) * 8;  // row 0 of this batch row
+        if constexpr (K::N % 2 == 0) {
+            // a full tile without self-mirrored rows, 16-byte aligned
+            constexpr int CPR = K::N / 2, C = K::P * CPR;
+            if (c.cnt == K::H && c.i0 > 0 && 2 * (c.i0 + K::H) <= n1 && (reinterpret_cast<uintptr_t>(ybase) & 15) == 0 &&
+                C % T == 0) {
+                const float2* y = reinterpret_cast<const float2*>(ybase);
+#pragma unroll
+                for (int i = 0; i < C / T; ++i) {
+                    const int slot = (tid + i * T) / CPR, cc = (tid + i * T) % CPR;
+                    const int row = slot < K::H ? c.i0 + slot : n1 - c.i0 + K::H - slot;
+                    sk_copy16(stage + slot * K::N + 2 * cc, y + (long long)row * K::N + 2 * cc);
+                }
+                return;
+            }
+        }
         // 16-byte copies when the rows are 16-byte aligned (a workspace from
         // cudaMalloc), 8-byte copies otherwise
         const int g = ((reinterpret_cast<uintptr_t>(ybase) | reinterpret_cast<uintptr_t>(stage)) & 15) == 0 ? 16 : 8;
@@ -1287,7 +1303,7 @@ SIP_HD void sk_pair_last_r2c_4b(int tid, const TileArgs& a, const TileCtx& c, co
         const float2* rb = buf + (self ? q : H + q) * K::LD;
         float2 A[R], B[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) A[r] = ra[K::idx(j + r * NR)];
+        for (int r = 0; r < R; ++r) A[r] = ra[K::last_slot(j, r)];
         if (j != 0) {
             float2 w[R];
             sk_pass_twiddles<K, PASS>(a, c, j, w);
@@ -1296,7 +1312,7 @@ SIP_HD void sk_pair_last_r2c_4b(int tid, const TileArgs& a, const TileCtx& c, co
         }
         dft<R, K::SIGN>(A);
 #pragma unroll
-        for (int r = 0; r < R; ++r) B[r] = rb[K::idx(jb + r * NR)];
+        for (int r = 0; r < R; ++r) B[r] = rb[K::last_slot(jb, r)];
         if (jb != 0) {
             float2 w[R];
             sk_pass_twiddles<K, PASS>(a, c, jb, w);
@@ -1825,6 +1841,8 @@ SIP_HD void sk_ip_last(int tid, const TileArgs& a, const TileCtx& c, const float
         sk_pair_last_r2c<K>(tid, a, c, buf);
     } else if constexpr (K::OP == OP_R2C_PAIR) {
         sk_pair_last_r2c_rows<K>(tid, a, c, buf);
+    } else if constexpr (K::OP == OP_R2C_4B) {
+        sk_pair_last_r2c_4b<K>(tid, a, c, buf);
     } else {
         using SP = SkPass<K, K::NP - 1>;
 #pragma unroll
