@@ -752,9 +752,11 @@ SIP_HD float2 sk_input(const TileArgs& a, const TileCtx& c, const float2* stage,
         return make_float2(s[(2 * q) * N + n], second ? s[(2 * q + 1) * N + n] : 0.f);
     }
     if constexpr (K::OP == OP_PC) {
-        if (a.flags & TF_BLUE) {  // Bluestein: chirp times the input, zero padded
-            const int nb = a.n_other;
-            return n < nb ? c_mul(stage[q * nb + n], SIP_LDG(a.tw2 + n)) : make_float2(0.f, 0.f);
+        if constexpr (!K::INPLACE) {  // (an in-place tile's read_slot does this itself)
+            if (a.flags & TF_BLUE) {  // Bluestein: chirp times the input, zero padded
+                const int nb = a.n_other;
+                return n < nb ? c_mul(stage[q * nb + n], SIP_LDG(a.tw2 + n)) : make_float2(0.f, 0.f);
+            }
         }
         return stage[q * N + n];
     } else if constexpr (K::OP == OP_C2C) {
@@ -895,6 +897,29 @@ struct SkPass {
                 return true;
             }
         }
+        if constexpr (PASS == 0 && !K::WORK_IN && K::INPLACE && K::OP == OP_PC && !K::TW4) {
+            if (a.flags & TF_BLUE) {
+                // Bluestein: inputs n < n_other <= (N + 1) / 2 times the chirp,
+                // both loads of every element before the products
+                constexpr int RH = R / 2 + 1;
+                const int nb = a.n_other;
+                const float2* x = buf + q * nb + j;
+                const float2* w = a.tw2 + j;
+                float2 h[RH];
+#pragma unroll
+                for (int r = 0; r < RH; ++r) {
+                    const bool in = j + r * NR < nb;
+                    v[r] = in ? x[r * NR] : make_float2(0.f, 0.f);
+                    h[r] = in ? SIP_LDG(w + r * NR) : make_float2(0.f, 0.f);
+                }
+#pragma unroll
+                for (int r = 0; r < RH; ++r) v[r] = c_mul(v[r], h[r]);
+#pragma unroll
+                for (int r = RH; r < R; ++r) v[r] = make_float2(0.f, 0.f);
+                dft<R, K::SIGN>(v);
+                return true;
+            }
+        }
         if constexpr (PASS == 0 && !K::WORK_IN && K::OP == OP_C2R_HALF) {
             // C2R pre-process: the twiddle of element n = j + r NR is
             // W_{2M}^{j + r NR} = W_{2M}^j W_{2R}^r, one table entry per
@@ -981,7 +1006,7 @@ struct SkPass {
         butterfly_index(b, q, j);
         if (!K::MIRROR && q >= c.cnt) return;
         if constexpr (K::OP == OP_C2C) {
-            const bool blue = K::WORK_IN && (a.flags & TF_BLUE) != 0;
+            const bool blue = K::WORK_IN && !K::INPLACE && (a.flags & TF_BLUE) != 0;
             if constexpr (K::TW4) sk_cross<K, R, NR>(a, c, q, j, v);
             if (blue) {  // Bluestein: outputs k < n_other times the chirp
 #pragma unroll
@@ -1924,6 +1949,26 @@ SIP_HD void sk_ip_inverse(int tid, const TileArgs& a, const TileCtx& c, float2* 
         if (q >= c.cnt) continue;
         float2* p = buf + SP::ip_slot(q, j);
         float2 v[R];
+        if constexpr (PASS == 0 && !K::TW4) {
+            if (a.flags & TF_BLUE) {
+                // Bluestein: outputs k < n_other <= (N + 1) / 2 times the chirp,
+                // whose loads start before the butterfly
+                constexpr int RH = R / 2 + 1;
+                float2 h[RH];
+                const float2* w = a.tw2 + j;
+#pragma unroll
+                for (int r = 0; r < RH; ++r)
+                    h[r] = j + r * SP::NR < a.n_other ? SIP_LDG(w + r * SP::NR) : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = p[r * K::ip_step(PASS)];
+                dft<R, 1>(v);
+                float2* d = static_cast<float2*>(a.dst) + c.out_base + (long long)q * a.out_idist + j;
+#pragma unroll
+                for (int r = 0; r < RH; ++r)
+                    if (j + r * SP::NR < a.n_other) d[r * SP::NR] = c_scale(c_mul(v[r], h[r]), a.scale);
+                continue;
+            }
+        }
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = p[r * K::ip_step(PASS)];
         dft<R, 1>(v);
