@@ -352,6 +352,22 @@ const std::vector<SkEntry>& sk_registry() {
         SIP_EMU_SK(0, 2025, 2, 128, OP_PC, SK_ROWS, 1, false, 1, 4, 19, 15, 15, 9)
         SIP_EMU_SK(0, 512, 8, 128, OP_PC, SK_ROWS, 1, true, 1, 4, 17, 32, 16)
         SIP_EMU_SK(0, 225, 16, 128, OP_PC, SK_ROWS, 1, true, 1, 4, 17, 15, 15)
+        // In-place tiles (SK_IN_PLACE) as the run-time compiler makes them, at
+        // lengths with no compiled kernel: staged and direct rows, columns of
+        // four, real halves and row pairs (tests/test_emu_in_place.py), and the
+        // passes of 256 x 256 as variants of the compiled ones.
+        SIP_EMU_SK(0, 1320, 3, 160, OP_C2C, SK_ROWS, -1, false, 2, 3, 27, 12, 11, 10)
+        SIP_EMU_SK(0, 1320, 3, 160, OP_C2C, SK_ROWS, 1, false, 2, 3, 25, 11, 10, 12)
+        SIP_EMU_SK(0, 1155, 2, 96, OP_C2C, SK_ROWS, -1, false, 1, 1, 17, 11, 7, 15)
+        SIP_EMU_SK(0, 1155, 1, 64, OP_C2C, SK_ROWS, 1, false, 1, 1, 19, 3, 5, 7, 11)
+        SIP_EMU_SK(0, 390, 4, 96, OP_C2C, SK_COLS, 1, false, 2, 1, 27, 6, 5, 13)
+        SIP_EMU_SK(0, 390, 3, 96, OP_C2C, SK_COLS, -1, false, 1, 1, 17, 13, 30)
+        SIP_EMU_SK(0, 256, 16, 128, OP_C2C, SK_COLS, -1, true, 2, 1, 27, 8, 4, 8)
+        SIP_EMU_SK(0, 256, 16, 128, OP_C2C, SK_ROWS_T, -1, false, 2, 1, 27, 4, 8, 8)
+        SIP_EMU_SK(0, 390, 3, 96, OP_R2C_HALF, SK_ROWS, -1, false, 2, 1, 31, 6, 5, 13)
+        SIP_EMU_SK(0, 390, 3, 96, OP_C2R_HALF, SK_ROWS, 1, false, 2, 1, 27, 6, 5, 13)
+        SIP_EMU_SK(0, 715, 2, 96, OP_R2C_PAIR, SK_ROWS, -1, false, 2, 1, 31, 13, 11, 5)
+        SIP_EMU_SK(0, 715, 2, 96, OP_C2R_PAIR, SK_ROWS, 1, false, 2, 1, 27, 13, 11, 5)
         // The self-sorting form (the library's for one-pass lengths) as variant 1.
         SIP_EMU_SK(0, 1000, 4, 128, OP_PC, SK_ROWS, 1, false, 2, 4, 1, 10, 10, 10)
         SIP_EMU_SK(0, 2025, 2, 192, OP_PC, SK_ROWS, 1, false, 2, 2, 1, 15, 15, 9)
