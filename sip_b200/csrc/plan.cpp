@@ -245,7 +245,7 @@ void try_specialize(Step& st, const AxisIO& io) {
     // A row step of less than one wave of tiles (two per SM) takes the
     // compiled variant with more threads per tile when there is one: each
     // transform's loads, passes and stores spread over more warps (C2C 4096
-    // x 256: 7.2 us with 256 threads per transform, 8.7 us with 128).
+    // x 256: 5.1 us with 256 threads per transform, in place, 6.3 us with 128).
     if (g_hint_variant < 0 && mode == SK_ROWS && !e->jit) {
         const long long tiles = (io.inner + e->P - 1) / e->P * io.outer;
         if (tiles <= kOneWaveTiles)
@@ -1015,12 +1015,14 @@ void add_real_large(FftPlan& plan, bool r2c, long long n, long long rows, Loc c2
     const bool split = four_step_split(m, &n1, &n2);
     const bool generic_only = std::getenv("SIP_FFT_GENERIC_ONLY") != nullptr || g_hint_generic;
     // C2R stays unfused by default: its fused pass A, with the pre-process on
-    // mirrored butterfly pairs too, measured slower (1.38 ms against 0.45 +
-    // 0.60 ms for 2^20 x 256); the real-fused and variant hints select it.
+    // mirrored butterfly pairs too, measured slower (1.38 ms for 2^20 x 256 when
+    // the two passes it replaces took 1.04 ms; they now take 0.32 + 0.44); the
+    // real-fused and variant hints select it.
     const bool fuse = g_hint_real_fused == 1 || (g_hint_real_fused == 0 && r2c);
     // R2C without a variant hint: the split whose pass B has the post-process
-    // on mirrored butterfly pairs (rows of 512 for m = 2^19: 1.36 ms for
-    // 2^20 x 256 against 1.46 with the 512 x 1024 split's pass B, which
+    // on mirrored butterfly pairs (rows of 512 for m = 2^19, in
+    // place with the next rows staged: 1.00 ms for 2^20 x 256 in whole passes;
+    // the 512 x 1024 split was 0.1 ms behind before that, as its pass B
     // holds 16 rows of 1024 in one CTA per SM)
     const SkEntry* pair_b = nullptr;
     if (split && !generic_only && fuse && r2c && g_hint_variant < 0 && !std::getenv("SIP_FFT_SPLIT_N1")) {

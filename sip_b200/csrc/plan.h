@@ -171,8 +171,10 @@ struct FftPlan {
     void* noalloc_scratch = nullptr;
     std::vector<Step> steps;
     std::vector<ChunkGroup> chunk_groups;
-    // Second stream and fork / join events of the two chunk lanes (made at
-    // device preparation when the plan has chunk groups).
+    // Second stream and fork / join events of the two chunk lanes: made at
+    // device preparation for units of 16 MB and more or a requested chunk size,
+    // with the second exec for the default chunks (plan.cpp
+    // size_default_chunks).
     mutable std::shared_ptr<ChunkLanes> lanes;
     mutable bool ran = false;  // an exec was launched (launch_steps)
 

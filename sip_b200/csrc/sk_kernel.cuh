@@ -16,6 +16,10 @@
 //   pass m-1:    registers -> global memory (coalesced), or -> shared memory
 //                followed by the real-transform post-process for R2C
 //
+// The self-sorting passes write to another place than they read; in-place
+// tiles (SK_IN_PLACE, "in-place passes" below) write a butterfly back where it
+// was, with one work buffer and the input staged beside it or read directly.
+//
 // Phase functions are __host__ __device__ and take (tid, T) so the CPU
 // harness (tests/native/tile_emu.cpp) runs them thread by thread.
 #pragma once
