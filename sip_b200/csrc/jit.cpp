@@ -155,15 +155,36 @@ std::vector<int> jit_pulse_radices(int n) {
     return best.empty() ? jit_radices(n) : best;
 }
 
+// Radices of an R2C tile: where the cheapest factorization has two passes
+// whose last is too wide for mirrored butterfly pairs in registers (above 21,
+// see sk_jit_choose), three with a last radix of 6 at most.  33.5 M values in
+// rows of 1400: 64 us as 14 x 10 x 5 on pairs against 74 as 28 x 25 without,
+// 1458 67 (27 x 9 x 3) against 84, 1536 59 (16 x 8 x 6) against 66.
+std::vector<int> jit_r2c_radices(int n) {
+    const std::vector<int> two = jit_radices(n);
+    if (two.size() != 2 || two.back() <= 21) return two;
+    for (int last = 6; last >= 3; --last) {
+        if (n % last != 0) continue;
+        std::vector<int> r = jit_radices(n / last);
+        if (r.size() != 2) continue;
+        r.push_back(last);
+        std::sort(r.begin(), r.end(), std::greater<int>());
+        return r;
+    }
+    return two;
+}
+
 // The factorization an operation's tiles use, found once per length (plans
 // are made per request by some programs).
 const std::vector<int>& tile_radices(int op, int n) {
     static std::mutex& mu = *new std::mutex;
-    static auto& known = *new std::map<std::pair<bool, int>, std::vector<int>>;
-    const auto key = std::make_pair(op == OP_PC, n);
+    static auto& known = *new std::map<std::pair<int, int>, std::vector<int>>;
+    const int kind = op == OP_PC ? 1 : op == OP_R2C_HALF || op == OP_R2C_PAIR ? 2 : 0;
+    const auto key = std::make_pair(kind, n);
     std::lock_guard<std::mutex> lk(mu);
     auto it = known.find(key);
-    if (it == known.end()) it = known.emplace(key, op == OP_PC ? jit_pulse_radices(n) : jit_radices(n)).first;
+    if (it == known.end())
+        it = known.emplace(key, kind == 1 ? jit_pulse_radices(n) : kind == 2 ? jit_r2c_radices(n) : jit_radices(n)).first;
     return it->second;
 }
 
@@ -343,8 +364,8 @@ bool sk_jit_choose(int op, int mode, int sign, bool tw4, int n, long long transf
     //    21 x 20: 94 us against 107).
     //  - R2C: in place too, on mirrored butterfly pairs, also for two passes
     //    whose pairs fit the registers (last radix up to 21): rows of 504
-    //    111 us against 144, 2400 126 against 183, 10000 134 against 191; 1250
-    //    as 25 x 25 150 self-sorting against 186.
+    //    111 us against 144, 2400 126 against 183, 10000 134 against 191 (67 M
+    //    values; 1250 as 25 x 25 150 self-sorting against 186).
     //  - C2R row pairs only above 5000 values (one tile of two rows is then
     //    most of an SM's shared memory): 6561 171 against 183, 12005 219
     //    against 288; 945 135 against 128, 3375 150 against 141.
