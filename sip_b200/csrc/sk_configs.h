@@ -91,7 +91,7 @@
     X(1, 2048, 1, 128, OP_C2R_HALF, SK_ROWS, 1, false, 2, 4, 15, 8, 16, 16)          \
     X(2, 4096, 1, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 2, 31, 16, 16, 16)       \
     X(3, 4096, 1, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 25, 16, 16, 16)        \
-    X(4, 1024, 4, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 3, 7, 16, 16, 4)          \
+    X(4, 1024, 4, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 2, 15, 16, 16, 4)        \
     X(5, 2048, 1, 128, OP_R2C_HALF, SK_ROWS, -1, false, 2, 4, 7, 16, 16, 8)          \
     X(6, 4096, 1, 256, OP_R2C_HALF, SK_ROWS, -1, false, 2, 2, 7, 16, 32, 8)          \
     /* 2D 500 x 50 (the reference's MRI example shape): rows of 50, columns \
@@ -141,6 +141,17 @@
     X(5, 1024, 4, 128, OP_C2C, SK_ROWS_T, 1, false, 2, 3, 9, 32, 32)                 \
     X(6, 256, 16, 256, OP_C2C, SK_COLS, -1, true, 2, 3, 9, 16, 16)                   \
     X(7, 256, 16, 256, OP_C2C, SK_COLS, 1, true, 2, 3, 9, 16, 16)                    \
+    /* forms for less than one wave of tiles, taken like the one below       \
+       (us, default form against these: C2C 1024 x 1024 5.8, 5.0, 8192 x 128  \
+       7.5, 5.9, R2C 2048 x 1024 7.7, 6.0, C2R 2048 x 1024 7.0, 5.7, C2R      \
+       6000 x 256 8.3, 6.3) */                                                \
+    X(6, 1024, 4, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 11, 16, 16, 4)          \
+    X(7, 2187, 1, 128, OP_C2R_PAIR, SK_ROWS, 1, false, 2, 4, 11, 27, 9, 9)           \
+    X(0, 3000, 1, 256, OP_C2R_HALF, SK_ROWS, 1, false, 2, 2, 11, 25, 8, 15)          \
+    X(1, 8192, 1, 256, OP_C2C, SK_ROWS, -1, false, 2, 1, 9, 32, 16, 16)              \
+    X(2, 8192, 1, 256, OP_C2C, SK_ROWS, 1, false, 2, 1, 9, 32, 16, 16)               \
+    X(4, 1024, 4, 256, OP_C2C, SK_ROWS, -1, false, 2, 2, 9, 16, 16, 4)               \
+    X(5, 1024, 4, 256, OP_C2C, SK_ROWS, 1, false, 2, 2, 9, 16, 16, 4)                \
     /* C2C 4096 rows, 256 threads per transform: taken automatically by row  \
        steps of less than one wave of tiles (plan.cpp try_specialize).  In    \
        place straight from global memory: one tile per CTA has nothing to    \

@@ -32,7 +32,9 @@ const SkEntry* sk_find(int op, int mode, int sign, bool tw4, int n, int variant 
 const SkEntry* sk_find_flags(int op, int mode, int sign, bool tw4, int n, int flags);
 
 // The first compiled variant of `e`'s kernel (same op, mode, sign, tw4, n
-// and transforms per tile) with more threads per tile; nullptr if none.
+// and transforms per tile) with more threads per tile, or with as many but
+// without staged twiddles where `e` stages them (a CTA that runs one tile
+// copies them for that tile alone); nullptr if none.
 const SkEntry* sk_find_wider(const SkEntry* e);
 
 const std::vector<SkEntry>& sk_registry();

@@ -398,7 +398,8 @@ const SkEntry* sk_find_flags(int op, int mode, int sign, bool tw4, int n, int fl
 const SkEntry* sk_find_wider(const SkEntry* e) {
     for (const SkEntry& x : sk_registry())
         if (x.op == e->op && x.mode == e->mode && x.sign == e->sign && x.tw4 == e->tw4 && x.n == e->n &&
-            x.P == e->P && x.T > e->T)
+            x.P == e->P &&
+            (x.T > e->T || (x.T == e->T && (e->flags & SK_TW_SMEM) != 0 && (x.flags & SK_TW_SMEM) == 0)))
             return &x;
     return nullptr;
 }
